@@ -1,5 +1,7 @@
-// Raw-DEFLATE inflate of BGZF members, one warp per member, with the CRC-32
-// of the output folded in.
+// Raw-DEFLATE inflate of BGZF members, with the CRC-32 of the output folded in.
+// Variant 0, the default, gives each member a CTA whose lanes all decode
+// (inflate_team.cuh).  The others, and what variant 0 falls back to, are the
+// serial form described here: one warp per member.
 //
 // A DEFLATE stream is a serial chain: a symbol's bit position is known only
 // once the previous symbol is decoded, and on GB300 one link of that chain --
@@ -75,6 +77,7 @@ template <int LB, int DB, u32 W, u32 Q, int R = 128, u32 S = 0> struct Cfg {
 struct CrcTables {
     u32 slice[4][256];
     u32 xpow[MAX_WB + 1];
+    u32 xpow4k[17]; // x^(8 * 4096 k): with xpow, every length up to 64 KiB
 };
 
 constexpr CrcTables make_crc_tables()
@@ -88,8 +91,9 @@ constexpr CrcTables make_crc_tables()
     for (int k = 1; k < 4; ++k)
         for (u32 i = 0; i < 256; ++i) t.slice[k][i] = (t.slice[k - 1][i] >> 8) ^ t.slice[0][t.slice[k - 1][i] & 0xffu];
     u32 v = 0x80000000u;
-    for (u32 m = 0; m <= MAX_WB; ++m) {
-        t.xpow[m] = v;
+    for (u32 m = 0; m <= 65536u; ++m) {
+        if (m <= MAX_WB) t.xpow[m] = v;
+        if (m % 4096u == 0) t.xpow4k[m / 4096u] = v;
         for (int k = 0; k < 8; ++k) v = (v >> 1) ^ (0xEDB88320u & (0u - (v & 1u)));
     }
     return t;
@@ -1293,6 +1297,8 @@ k_inflate_persistent_multi(const u8 *in, const u64 *in_off, const u32 *in_len, u
                               crc_expect, status, produced, crc, order, n, out_capacity, queue_head, block_err, 0u);
 }
 
+#include "inflate_team.cuh"
+
 } // namespace
 
 // Standalone CRC of already-inflated members (the reference's crc32_blocks,
@@ -1335,28 +1341,41 @@ struct Variant {
     frt_inflate_variant info;
     MembersKernel members;
     PersistentKernel persistent;
+    u32 team; // warps that share one member, the CTA of a team variant; 0: a warp has members of its own
 };
 
 template <class C> Variant make_variant()
 {
     return {{C::LIT_BITS, C::DIST_BITS, (int32_t)C::WB, (int32_t)C::MAXQ, C::REGS, 1, (int32_t)C::STAGE,
              (uint64_t)warp_smem_bytes<C>()},
-            k_inflate_members<C>, k_inflate_persistent<C>};
+            k_inflate_members<C>, k_inflate_persistent<C>, 0u};
 }
 
 template <class C, int K> Variant make_multi_variant()
 {
     return {{C::LIT_BITS, C::DIST_BITS, (int32_t)C::WB, (int32_t)C::MAXQ, C::REGS, K, (int32_t)C::STAGE,
              (uint64_t)multi_warp_bytes<C, K>()},
-            k_inflate_members_multi<C, K>, k_inflate_persistent_multi<C, K>};
+            k_inflate_members_multi<C, K>, k_inflate_persistent_multi<C, K>, 0u};
+}
+
+// A team variant's shape is given per warp of the team, whose warps share one
+// output buffer and one match list.
+template <int NW, int PER_SM> Variant make_team_variant()
+{
+    using S = team::Smem<NW>;
+    return {{(int32_t)team::LR, (int32_t)team::DR, (int32_t)((team::OUT_MAX / NW + 31) / 32 * 32), (int32_t)team::GROUP_MATCHES,
+             65536 / (32 * NW * PER_SM) / 8 * 8, 1, 0, (uint64_t)((sizeof(S) + NW - 1) / NW)},
+            team::k_members<NW, PER_SM>, team::k_persistent<NW, PER_SM>, (u32)NW};
 }
 
 // The compiled variants: the table roots trade shared memory (members in
 // flight) against codes that take the long path; the window buffer and its
 // queue trade shared memory against bursts per member; a register cap (80:
 // no spills; 72, 64 and 56: up to ~120 spilled bytes) lets more CTAs fit an SM.
-// Variant 0 is the default before any tuning.
+// Variant 0 is the default before any tuning: the team form, one member per
+// CTA whatever CTA width a tuning names.
 const Variant kVariants[] = {
+    make_team_variant<12, 2>(),
     make_variant<Cfg<10, 8, 2048, 384>>(),     make_variant<Cfg<9, 8, 2048, 384>>(),
     make_variant<Cfg<11, 8, 2048, 384>>(),     make_variant<Cfg<10, 8, 1024, 256>>(),
     make_variant<Cfg<9, 7, 1024, 256>>(),      make_variant<Cfg<10, 8, 4096, 768>>(),
@@ -1387,6 +1406,8 @@ extern "C" int frt_inflate_variant_count(void) { return kNumVariants; }
 
 const frt_inflate_variant *frt_inflate_variant_at(int v) { return v >= 0 && v < kNumVariants ? &kVariants[v].info : nullptr; }
 
+int frt::inflate_variant_team(int v) { return v >= 0 && v < kNumVariants ? (int)kVariants[v].team : 0; }
+
 extern "C" int frt_inflate_variant_info(int32_t variant, frt_inflate_variant *out, frt_error *err)
 {
     if (!out || variant < 0 || variant >= kNumVariants) {
@@ -1410,8 +1431,18 @@ void frt_inflate_set_default(const frt_inflate_tuning &t)
     g_tuning = t;
 }
 
+namespace {
+u32 cta_threads(const frt_inflate_tuning &t)
+{
+    const u32 team = kVariants[t.variant].team;
+    return 32u * (team ? team : (u32)t.warps_per_cta);
+}
+} // namespace
+
 size_t frt_inflate_smem_bytes(const frt_inflate_tuning &t)
 {
+    const u32 team = kVariants[t.variant].team;
+    if (team) return (size_t)team * kVariants[t.variant].info.smem_per_warp;
     return (size_t)t.warps_per_cta * kVariants[t.variant].info.smem_per_warp;
 }
 
@@ -1437,7 +1468,7 @@ int frt_inflate_ctas_per_sm(const frt_inflate_tuning &t)
         t.spread_variant >= kNumVariants || (t.spread_variant >= 0 && kVariants[t.spread_variant].info.chains != 1))
         return 0;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kVariants[t.variant].persistent, t.warps_per_cta * 32,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kVariants[t.variant].persistent, (int)cta_threads(t),
                                                       frt_inflate_smem_bytes(t)) != cudaSuccess)
         return 0;
     if (t.ctas_per_sm > 0 && t.ctas_per_sm < per_sm) per_sm = t.ctas_per_sm;
@@ -1492,7 +1523,7 @@ bool spread_launch(frt_inflate_tuning &t, u64 n, u32 *grid)
 {
     const int v = t.spread_variant >= 0 ? t.spread_variant : t.variant;
     if (kVariants[v].info.chains != 1 || n == 0) return false;
-    if (t.warps_per_cta <= 1 && v == t.variant) return false;
+    if ((t.warps_per_cta <= 1 || kVariants[v].team) && v == t.variant) return false;
     int per_sm = g_spread_ctas[v].load(std::memory_order_relaxed);
     if (per_sm == 0) {
         frt_inflate_tuning one{v, 1, 0, 1, -1};
@@ -1517,8 +1548,8 @@ cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u3
     frt_inflate_tuning t = tuned;
     u32 unused = 0;
     spread_launch(t, n, &unused);
-    const u32 w = (u32)t.warps_per_cta * (u32)kVariants[t.variant].info.chains; // members per CTA
-    kVariants[t.variant].members<<<(n + w - 1) / w, t.warps_per_cta * 32, frt_inflate_smem_bytes(t), s>>>(
+    const u32 w = kVariants[t.variant].team ? 1u : (u32)t.warps_per_cta * (u32)kVariants[t.variant].info.chains; // members per CTA
+    kVariants[t.variant].members<<<(n + w - 1) / w, cta_threads(t), frt_inflate_smem_bytes(t), s>>>(
         in, in_off, in_len, out, out_off, out_cap, status, produced, crc, n);
     return cudaGetLastError();
 }
@@ -1532,8 +1563,10 @@ cudaError_t frt_launch_inflate_persistent(const u8 *in, const u64 *in_off, const
     // n_cap bounds the members (the device count may be lower): fewer than
     // the tuned grid's warps gives a spread launch of n_cap one-warp CTAs
     frt_inflate_tuning t = tuned;
-    if (n_cap < (u64)grid * (u64)tuned.warps_per_cta) spread_launch(t, n_cap, &grid);
-    kVariants[t.variant].persistent<<<grid, t.warps_per_cta * 32, frt_inflate_smem_bytes(t), s>>>(
+    // (a team variant needs no spreading: a CTA per member at most)
+    if (kVariants[t.variant].team && n_cap < grid) grid = (u32)(n_cap ? n_cap : 1);
+    else if (n_cap < (u64)grid * (u64)tuned.warps_per_cta) spread_launch(t, n_cap, &grid);
+    kVariants[t.variant].persistent<<<grid, cta_threads(t), frt_inflate_smem_bytes(t), s>>>(
         in, in_off, in_len, out, out_off, isize, crc_expect, status, produced, crc, order, n_ptr, n_cap,
         out_capacity, queue_head, (u32)t.queue_chunk, block_err);
     return cudaGetLastError();

@@ -114,4 +114,7 @@ namespace frt {
 void batch_release(const frt_inflate_batch *b);
 int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const frt_span *spans, size_t n,
                   frt_inflate_batch **out, frt_error *err);
+// Warps that share one member in a team variant of the inflate (its CTA,
+// whatever CTA width a tuning names); 0 where each warp has its own members.
+int inflate_variant_team(int variant);
 } // namespace frt

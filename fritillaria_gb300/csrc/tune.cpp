@@ -560,6 +560,7 @@ extern "C" int frt_autotune(frt_engine *e, const char *cache_path, int32_t force
     static const int widths[] = {2, 3, 4, 6, 8};
     for (int v = 0; v < frt_inflate_variant_count(); ++v)
         for (int w : widths) {
+            if (frt::inflate_variant_team(v) && w != widths[0]) continue; // its CTA is the team, whatever the width
             frt_inflate_tuning t{v, w, 0, 1, -1};
             if (t.variant == cur.variant && t.warps_per_cta == cur.warps_per_cta && cur.ctas_per_sm == 0 &&
                 cur.queue_chunk == 1)

@@ -609,7 +609,8 @@ void frt_server_release(frt_server *s, uint64_t request);
  * set and workload class. */
 typedef struct {
     int32_t variant;        /* index of a compiled variant */
-    int32_t warps_per_cta;  /* 1..8; each warp takes the variant's chains of members */
+    int32_t warps_per_cta;  /* 1..8; each warp takes the variant's chains of members (variant 0, the
+                               team form, gives a member a CTA of its own width whatever this says) */
     int32_t ctas_per_sm;    /* 0: as many as fit */
     int32_t queue_chunk;    /* members per queue pop, 1..64 */
     int32_t spread_variant; /* -1, or a one-chain variant for small launches: a launch of fewer members
@@ -621,8 +622,8 @@ typedef struct {
 typedef struct {
     int32_t lit_bits;       /* literal/length table root */
     int32_t dist_bits;      /* distance table root */
-    int32_t window;         /* window buffer per warp, bytes */
-    int32_t queue;          /* matches queued per window */
+    int32_t window;         /* window buffer per warp, bytes (team form: its share of the member's output) */
+    int32_t queue;          /* matches queued per window (team form: listed per 256 bytes) */
     int32_t max_registers;  /* register cap per thread */
     int32_t chains;         /* members a warp decodes side by side, one lane each */
     int32_t stage_half;     /* 0: compressed bytes read through L1; else the bytes of each half of a

@@ -1,0 +1,68 @@
+"""The team form of the inflate (one CTA per member, every lane decoding) at the
+sizes where it can go wrong: empty and one-byte members, a member of exactly
+64 KiB, match lists past their room, blocks of a few bits and
+of one segment, many blocks a member, second-level codes, stored runs between
+coded blocks, and outputs at every alignment -- the bytes zlib gives back."""
+
+import zlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _content(kind: str, n: int, rng) -> bytes:
+    if kind == "zeros":
+        return bytes(n)
+    if kind == "period":  # distances shorter than a match, 1 to 40 bytes
+        out = bytearray()
+        while len(out) < n:
+            unit = bytes(rng.integers(0, 256, int(rng.integers(1, 41)), dtype=np.uint8))
+            out += unit * int(rng.integers(2, 30))
+        return bytes(out[:n])
+    if kind == "pairs":  # three-byte matches as dense as they come: the match list overflows
+        words = [bytes(rng.integers(0, 256, 3, dtype=np.uint8)) for _ in range(300)]
+        return b"".join(words[i] for i in rng.integers(0, 300, n // 3 + 1))[:n]
+    if kind == "skewed":  # code lengths up to 15 bits: second-level tables
+        p = 0.6 ** np.arange(60)
+        return bytes(rng.choice(60, n, p=p / p.sum()).astype(np.uint8) * 4)
+    if kind == "noise":
+        return bytes(rng.integers(0, 256, n, dtype=np.uint8))
+    half = n // 2  # "mixed": text, then noise (a stored block between coded ones)
+    text = b"".join(b"chr%d\t%d\t%s\n" % (i % 23, i * 37, b"ACGT"[i % 4:i % 4 + 1] * (i % 9)) for i in range(half // 8 + 1))
+    return text[:half] + bytes(rng.integers(0, 256, n - half, dtype=np.uint8))
+
+
+SIZES = [0, 1, 2, 3, 15, 16, 17, 255, 4096, 12287, 12289, 32768, 65280, 65535, 65536]
+
+
+def _file(streams):
+    """The streams back to back at odd distances, and their spans."""
+    from fritillaria_gb300 import SPAN_DTYPE
+
+    data, spans = bytearray(b"\x55" * 5), []
+    for k, (payload, raw) in enumerate(streams):
+        spans.append((len(data), len(data), len(payload), len(raw), zlib.crc32(raw)))
+        data += payload + b"\xaa" * (8 + k % 7)
+    return np.frombuffer(bytes(data), np.uint8), np.array(spans, dtype=SPAN_DTYPE)
+
+
+def _deflate(raw, level, strategy=zlib.Z_DEFAULT_STRATEGY, mem=8):
+    co = zlib.compressobj(level, zlib.DEFLATED, -15, mem, strategy)
+    return co.compress(raw) + co.flush()
+
+
+@pytest.mark.parametrize("kind", ["zeros", "period", "pairs", "skewed", "noise", "mixed"])
+def test_edges_equal_zlib(gpu, kind):
+    rng = np.random.default_rng(len(kind))
+    assert gpu.default_tuning().variant == 0
+    streams = []
+    for n in SIZES:
+        raw = _content(kind, n, rng)
+        for level, strategy, mem in ((1, 0, 8), (6, 0, 8), (9, 0, 1), (6, zlib.Z_HUFFMAN_ONLY, 8), (6, zlib.Z_FIXED, 9), (0, 0, 8)):
+            streams.append((_deflate(raw, level, strategy, mem), raw))
+    data, spans = _file(streams)
+    got, offs = gpu.CudaCodec(0).inflate_batch(data, spans)
+    for i, (_, raw) in enumerate(streams):
+        assert got[offs[i]:offs[i + 1]].tobytes() == raw, (kind, i)
