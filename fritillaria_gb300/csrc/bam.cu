@@ -7,11 +7,12 @@
 // (crates/fritillaria-cuda/kernels/bam_decode.cu:154-216).  This file removes
 // that serial walk:
 //
-//   1. spec: one warp per member searches the member for its first plausible
-//      record start (a 32-offset sieve with a strict validator: block_size,
+//   1. spec: a CTA per member searches the member for its first plausible
+//      record start (a 512-offset sieve with a strict validator: block_size,
 //      refID/next_refID range, positions, NUL-terminated name, declared fields
-//      fit, and the following record validates too) and walks the chain from
-//      there to the member end, recording record offsets in scratch;
+//      fit, and the next two records validate too) and walks the chain from
+//      there to the member end, recording record offsets in scratch -- an
+//      eighth of the member a warp, the parts joined where walks meet;
 //   2. reconcile: one CTA proves the chain.  The true arrival into member m is
 //      max(start, lands of earlier members that hold a record start) -- a
 //      prefix max, computed block-wide.  Member m is proven when its
@@ -121,41 +122,39 @@ __device__ Seg walk_record(const u8 *buf, u64 len, u64 from, u64 until, u64 msta
 
 } // namespace
 
-// Phase 1 for member m: the first plausible record start, then the walk to
-// the member end.  Called by one whole warp.
-__device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u64 start, int n_ref, u64 *entry,
-                            u32 *count, u64 *land, u8 *flags, u16 *scratch)
+// The first plausible record start in [lo, hi), whose two next records are
+// plausible too (wherever they fall in the batch: a decoy's length usually
+// lands far away), or INF64.  By one warp.
+//
+// 512 offsets a turn, four groups of four a lane, their loads in flight
+// together.  plausible() needs ref_id in [-1, n_ref), which random bytes almost
+// never hold, so each lane first builds its ref_id words from aligned word
+// loads and runs the full test only where that passes.  A word outside [0, len)
+// reads as 0 (the full test then rejects the offset: its header would pass
+// len); the ref_id words of any offset with a whole header lie inside.
+__device__ u64 find_start(const u8 *buf, u64 len, u64 lo, u64 hi, int n_ref)
 {
     const u32 lane = lane_id();
-    u64 ms = starts[m], me = starts[m + 1];
-    u64 e = INF64;
-    if (me <= start) {
-        // entirely before the first record: nothing starts here
-    } else if (ms <= start) {
-        e = start;
-    } else {
-        // 128 offsets a turn, four a lane.  plausible() needs ref_id in
-        // [-1, n_ref), which random bytes almost never hold, so each lane first
-        // builds its four ref_id words from two aligned word loads and runs the
-        // full test only where that passes.  A word outside [0, len) reads as 0
-        // (the full test then rejects the offset: its header would pass len);
-        // the ref_id words of any offset with a whole header lie inside.
-        const long long A = (long long)(((uintptr_t)(buf + ms) & ~(uintptr_t)3) - (uintptr_t)buf);
-        for (long long base = A; base < (long long)me; base += 128) {
-            const long long wo = base + 4ll * lane + 4ll;
-            const u32 w0 = wo >= 0 && wo + 4 <= (long long)len ? *(const u32 *)(buf + wo) : 0u;
-            const u32 w1 = wo + 4 >= 0 && wo + 8 <= (long long)len ? *(const u32 *)(buf + wo + 4) : 0u;
+    const long long A = (long long)(((uintptr_t)(buf + lo) & ~(uintptr_t)3) - (uintptr_t)buf);
+    for (long long base = A; base < (long long)hi; base += 512) {
+        u32 w0[4], w1[4];
+#pragma unroll
+        for (u32 g = 0; g < 4u; ++g) {
+            const long long wo = base + 128 * g + 4ll * lane + 4ll;
+            w0[g] = wo >= 0 && wo + 4 <= (long long)len ? *(const u32 *)(buf + wo) : 0u;
+            w1[g] = wo + 4 >= 0 && wo + 8 <= (long long)len ? *(const u32 *)(buf + wo + 4) : 0u;
+        }
+#pragma unroll
+        for (u32 g = 0; g < 4u; ++g) {
             u32 first = 4;
 #pragma unroll
             for (u32 k = 0; k < 4u; ++k) {
-                const u32 ref = k ? __funnelshift_r(w0, w1, 8u * k) : w0;
-                const long long ps = base + 4ll * lane + k;
-                if (first == 4 && ps >= (long long)ms && ps < (long long)me && ref + 1u <= (u32)n_ref) {
+                const u32 ref = k ? __funnelshift_r(w0[g], w1[g], 8u * k) : w0[g];
+                const long long ps = base + 128 * g + 4ll * lane + k;
+                if (first == 4 && ps >= (long long)lo && ps < (long long)hi && ref + 1u <= (u32)n_ref) {
                     const u64 p = (u64)ps;
                     bool ok = plausible(buf, len, p, n_ref);
                     if (ok) {
-                        // the next two records must validate as well, wherever they
-                        // fall in the batch (a decoy's length usually lands far away)
                         u64 q = p + 4ull + ld_u32le(buf + p);
                         for (int j = 0; j < 2 && ok && q + 36 <= len; ++j) {
                             ok = plausible(buf, len, q, n_ref);
@@ -168,27 +167,93 @@ __device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u6
             const u32 hit = __ballot_sync(FRT_FULL_MASK, first < 4u);
             if (hit) {
                 const u32 src = (u32)(__ffs(hit) - 1);
-                e = (u64)(base + 4ll * src + __shfl_sync(FRT_FULL_MASK, first, src));
-                break;
+                return (u64)(base + 128 * g + 4ll * src + __shfl_sync(FRT_FULL_MASK, first, src));
             }
         }
     }
-    Seg s{e, 0u, 1, 1};
-    if (lane == 0 && e != INF64) s = walk_record(buf, len, e, me, ms, scratch + (size_t)m * FRT_SCAN_CAP, FRT_SCAN_CAP);
-    if (lane == 0) {
-        entry[m] = e;
-        count[m] = s.count;
-        land[m] = e == INF64 ? 0ull : s.land;
-        flags[m] = (u8)((s.complete ? 1 : 0) | (s.valid ? 2 : 0));
-    }
+    return INF64;
 }
 
-// Phase 1.  One warp per member.
-__global__ void k_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n_members, u64 start,
-                                        int n_ref, u64 *entry, u32 *count, u64 *land, u8 *flags, u16 *scratch,
-                                        const u64 *start_dev, const int *nref_dev)
+constexpr u32 SPEC_WARPS = 8;                          // parts of a member, a warp each
+constexpr u32 SPEC_PART = 65536 / SPEC_WARPS;          // most bytes of a part
+constexpr u32 SPEC_CAP = (SPEC_PART + 35) / 36;        // most record starts in one
+
+// Phase 1 for member m, by a CTA: the first plausible record start, then the
+// walk to the member end.
+//
+// A walk is a chain of loads, each record's place known only from the one
+// before: 220 short reads a member took 175 us whatever the file's size, and a
+// member of an ultra-long read that holds no start at all was searched 128
+// offsets at a time for 316 us.  So a warp takes an eighth of the member: it
+// searches its part and walks it from what it found.  One thread then follows
+// the walks from the member's first start: where a walk lands on the start its
+// part's warp found, that part's records are the chain's; elsewhere the part
+// is walked again from the landing.  The result is the one walk's.
+__device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u64 start, int n_ref, u64 *entry,
+                            u32 *count, u64 *land, u8 *flags, u16 *scratch)
 {
-    u32 m = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    __shared__ u64 s_entry[SPEC_WARPS], s_land[SPEC_WARPS];
+    __shared__ u32 s_count[SPEC_WARPS], s_flags[SPEC_WARPS];
+    __shared__ u16 s_rec[SPEC_WARPS][SPEC_CAP];
+    const u32 lane = lane_id(), w = threadIdx.x / 32;
+    const u64 ms = starts[m], me = starts[m + 1];
+    // a member past 64 KiB (none is) stays one part, walked into its place
+    const bool whole = me - ms > 65536;
+    const u64 part = whole ? me - ms : max((me - ms + SPEC_WARPS - 1) / SPEC_WARPS, (u64)1);
+    const u64 lo = min(me, ms + w * part), hi = min(me, lo + part);
+    u16 *const place = scratch + (size_t)m * FRT_SCAN_CAP;
+    u64 e = INF64;
+    if (lo < hi && hi > start) e = lo <= start ? start : find_start(buf, len, lo, hi, n_ref);
+    if (lane == 0) {
+        Seg s{e, 0u, 1, 1};
+        if (e != INF64) s = whole ? walk_record(buf, len, e, hi, ms, place, FRT_SCAN_CAP) : walk_record(buf, len, e, hi, ms, s_rec[w], SPEC_CAP);
+        s_entry[w] = e;
+        s_land[w] = s.land;
+        s_count[w] = s.count;
+        s_flags[w] = (s.complete ? 1u : 0u) | (s.valid ? 2u : 0u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        u64 cur = INF64, first = INF64, at = 0;
+        u32 k = 0, n = 0, f = 3;
+        while (k < SPEC_WARPS && s_entry[k] == INF64) s_count[k++] = 0;
+        if (k < SPEC_WARPS) first = cur = s_entry[k];
+        for (; k < SPEC_WARPS; ++k) {
+            const u64 end = min(me, ms + (k + 1) * part);
+            if (cur >= end) { // covered by a record that began before
+                s_count[k] = 0;
+                continue;
+            }
+            if (s_entry[k] != cur) {
+                const Seg s = walk_record(buf, len, cur, end, ms, s_rec[k], SPEC_CAP);
+                s_land[k] = s.land;
+                s_count[k] = s.count;
+                s_flags[k] = (s.complete ? 1u : 0u) | (s.valid ? 2u : 0u);
+            }
+            n += s_count[k];
+            cur = at = s_land[k];
+            f = s_flags[k];
+            if (f != 3u) break;
+        }
+        for (++k; k < SPEC_WARPS; ++k) s_count[k] = 0; // past a walk that stopped
+        entry[m] = first;
+        count[m] = n;
+        land[m] = first == INF64 ? 0ull : at;
+        flags[m] = (u8)f;
+    }
+    __syncthreads();
+    if (whole) return;
+    u32 before = 0;
+    for (u32 k = 0; k < w; ++k) before += s_count[k];
+    for (u32 i = lane; i < s_count[w]; i += 32) place[before + i] = s_rec[w][i];
+}
+
+// Phase 1.  One CTA per member.
+__global__ void __launch_bounds__(32 * SPEC_WARPS)
+k_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n_members, u64 start, int n_ref, u64 *entry, u32 *count,
+           u64 *land, u8 *flags, u16 *scratch, const u64 *start_dev, const int *nref_dev)
+{
+    u32 m = blockIdx.x;
     if (m >= n_members) return;
     if (start_dev) start = *start_dev;
     if (nref_dev) n_ref = *nref_dev < 0 ? (1 << 24) : *nref_dev;
@@ -198,10 +263,11 @@ __global__ void k_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n_memb
 // Phase 1 over many segments (independent record chains, each over its own
 // members): segment s owns members [seg[s].m0, seg[s].m0 + seg[s].n) of the
 // per-member arrays and the n + 1 starts at starts + seg[s].m0 + s.
-__global__ void k_bam_spec_seg(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_total, int n_ref,
-                               const u64 *starts, u64 *entry, u32 *count, u64 *land, u8 *flags, u16 *scratch)
+__global__ void __launch_bounds__(32 * SPEC_WARPS)
+k_bam_spec_seg(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_total, int n_ref, const u64 *starts,
+               u64 *entry, u32 *count, u64 *land, u8 *flags, u16 *scratch)
 {
-    u32 g = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    u32 g = blockIdx.x;
     if (g >= n_total) return;
     u32 si = seg_of[g];
     FrtScanSeg sg = seg[si];
@@ -720,7 +786,7 @@ cudaError_t frt_launch_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n
                                 const int *nref_dev)
 {
     if (n == 0) return cudaSuccess;
-    k_bam_spec<<<(n + 7) / 8, 256, 0, s>>>(buf, len, starts, n, start, n_ref, entry, count, land, flags, scratch,
+    k_bam_spec<<<n, 32 * SPEC_WARPS, 0, s>>>(buf, len, starts, n, start, n_ref, entry, count, land, flags, scratch,
                                            start_dev, nref_dev);
     return cudaGetLastError();
 }
@@ -750,8 +816,8 @@ cudaError_t frt_launch_region_scan(const u8 *buf, const FrtScanSeg *seg, const u
                                    u8 *flags, u16 *scratch, u32 *first_index, u64 *totals, u32 *kept, cudaStream_t s)
 {
     if (n_total == 0 || n_segs == 0) return cudaSuccess;
-    unsigned g = (n_total + 7) / 8;
-    k_bam_spec_seg<<<g, 256, 0, s>>>(buf, seg, seg_of, n_total, n_ref, starts, entry, count, land, flags, scratch);
+    unsigned g = (n_total + 7) / 8; // warp-per-member grids below
+    k_bam_spec_seg<<<n_total, 32 * SPEC_WARPS, 0, s>>>(buf, seg, seg_of, n_total, n_ref, starts, entry, count, land, flags, scratch);
     k_bam_reconcile_seg<<<n_segs, 1024, 0, s>>>(buf, seg, starts, entry, count, land, flags, scratch, first_index,
                                                 totals);
     k_region_count<<<g, 256, 0, s>>>(buf, seg, seg_of, n_total, starts, coff, count, scratch, kept);
