@@ -543,8 +543,6 @@ __global__ void k_region_emit(const u8 *buf, const FrtScanSeg *seg, const u32 *s
 
 namespace {
 
-// One aux field at `pos` (aux.rs:301-405): returns the offset just past it,
-// or 0 when malformed.  Fills type/subtype/value offset/count.
 // The first zero byte of rec[q, end), or end.  Long Z strings (MM:Z of an
 // ultra-long read runs to 100 KB) go 32 bytes a step through aligned 16-byte
 // loads; no load reaches past end.
@@ -567,18 +565,73 @@ __device__ __forceinline__ u32 find_nul(const u8 *rec, u32 q, u32 end)
     return end;
 }
 
-__device__ __forceinline__ u32 aux_field(const u8 *rec, u32 pos, u32 end, u32 *w0, u32 *voff, u32 *cnt)
+// The same for one lane's string by the whole warp (every argument the same in
+// all lanes): 2 KiB a turn, four 16-byte loads a lane in flight.  A lane alone
+// took 400 us over the 120 KB strings of the longest reads, twice a run.
+__device__ u32 find_nul_warp(const u8 *rec, u32 q, u32 end)
 {
-    if (pos + 3 > end) return 0;
-    u32 ty = rec[pos + 2];
-    u32 v = pos + 3;
+    const u32 lane = lane_id();
+    const uintptr_t from = (uintptr_t)(rec + q), stop = (uintptr_t)(rec + end);
+    for (uintptr_t base = from & ~(uintptr_t)15; base < stop; base += 2048) {
+        u32 z[4];
+#pragma unroll
+        for (u32 j = 0; j < 4; ++j) {
+            const uintptr_t a = base + 512 * j + 16 * lane;
+            u32 m = 0; // a bit for each byte of the block that is zero and in [q, end)
+            if (a >= from && a + 16 <= stop) {
+                const uint4 v = *(const uint4 *)a;
+                const u32 w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) m |= (((__vcmpeq4(w[k], 0u) & 0x08040201u) * 0x01010101u) >> 24) << (4 * k);
+            } else {
+                for (u32 b = 0; b < 16; ++b)
+                    if (a + b >= from && a + b < stop && *(const u8 *)(a + b) == 0) m |= 1u << b;
+            }
+            z[j] = m;
+        }
+#pragma unroll
+        for (u32 j = 0; j < 4; ++j) {
+            const u32 hit = __ballot_sync(FRT_FULL_MASK, z[j] != 0);
+            if (hit) {
+                const u32 l = __ffs(hit) - 1, b = __ffs(__shfl_sync(FRT_FULL_MASK, z[j], l)) - 1;
+                return (u32)(base + 512 * j + 16 * l + b - (uintptr_t)rec);
+            }
+        }
+    }
+    return end;
+}
+
+constexpr u32 NUL_ALONE = 64; // bytes of a string a lane looks at before the warp does
+
+// One aux field at `pos` (aux.rs:301-405) for every lane that is `on`, by the
+// whole warp: the offset just past it, or 0 when malformed.  Fills type and
+// tag, value offset and count.
+__device__ __forceinline__ u32 aux_field(bool on, const u8 *rec, u32 pos, u32 end, u32 *w0, u32 *voff, u32 *cnt)
+{
+    on = on && pos + 3 <= end;
+    const u32 v = pos + 3;
+    const u32 ty = on ? rec[pos + 2] : 0u;
+    const bool text = ty == 'Z' || ty == 'H';
+    u32 q = 0;
+    bool more = false;
+    if (text) {
+        const u32 lim = min(end, v + NUL_ALONE);
+        q = find_nul(rec, v, lim);
+        more = q >= lim && lim < end;
+    }
+    for (u32 m = __ballot_sync(FRT_FULL_MASK, more); m; m &= m - 1) {
+        const u32 l = __ffs(m) - 1;
+        const u8 *r = (const u8 *)(uintptr_t)__shfl_sync(FRT_FULL_MASK, (unsigned long long)(uintptr_t)rec, l);
+        const u32 found = find_nul_warp(r, __shfl_sync(FRT_FULL_MASK, v + NUL_ALONE, l), __shfl_sync(FRT_FULL_MASK, end, l));
+        if (lane_id() == l) q = found;
+    }
+    if (!on) return 0;
     u32 sub = 0, count = 1, next;
     switch (ty) {
     case 'A': case 'c': case 'C': next = v + 1; break;
     case 's': case 'S': next = v + 2; break;
     case 'i': case 'I': case 'f': next = v + 4; break;
     case 'Z': case 'H': {
-        const u32 q = find_nul(rec, v, end);
         if (q >= end) return 0;
         count = q - v;
         if (ty == 'H') {
@@ -632,52 +685,65 @@ __global__ void k_bam_decode(const u8 *buf, const u64 *starts, const u64 *member
     u64 vbase = member_coffset ? (member_coffset[m] << 16) : 0ull;
     u32 first = first_index[m];
     const u16 *rec = scratch + (size_t)m * FRT_SCAN_CAP;
-    for (u32 k = lane_id(); k < n; k += 32) {
-        u32 rel = rec[k];
-        u64 r = ms + rel;
-        const u8 *p = buf + r;
-        u64 i = (u64)first + k;
-        if (i >= rec_cap) break;
-        u32 bs = ld_u32le(p);
-        u32 name_len = p[12];
-        u32 n_cigar = ld_u16le(p + 16);
-        u32 l_seq = ld_u32le(p + 20);
-        c.ref_id[i] = (int)ld_u32le(p + 4);
-        c.pos[i] = (int)ld_u32le(p + 8);
-        c.name_len[i] = (u8)name_len;
-        c.mapq[i] = p[13];
-        c.bin[i] = (u16)ld_u16le(p + 14);
-        c.n_cigar[i] = (u16)n_cigar;
-        c.flags[i] = (u16)ld_u16le(p + 18);
-        c.seq_len[i] = l_seq;
-        c.mate_ref_id[i] = (int)ld_u32le(p + 24);
-        c.mate_pos[i] = (int)ld_u32le(p + 28);
-        c.tlen[i] = (int)ld_u32le(p + 32);
-        c.record_offsets[i] = r;
-        c.virtual_offset[i] = vbase | rel;
-        u32 cs = 36u + name_len;
-        u32 ss = cs + 4u * n_cigar;
-        u32 qs = ss + (l_seq + 1u) / 2u;
-        u32 as = qs + l_seq;
-        u32 re = 4u + bs;
-        c.cigar_start[i] = cs;
-        c.sequence_start[i] = ss;
-        c.quality_start[i] = qs;
-        c.aux_start[i] = as;
-        c.record_end[i] = re;
-        u32 nt = 0, st = 0, pos = as;
-        while (pos < re) {
-            u32 w0, vo, cn;
-            u32 nx = aux_field(p, pos, re, &w0, &vo, &cn);
-            if (!nx) {
-                st = 1;
-                break;
-            }
-            ++nt;
-            pos = nx;
+    for (u32 k0 = 0; k0 < n; k0 += 32) {
+        const u32 k = k0 + lane_id();
+        const u64 i = (u64)first + k;
+        const bool on = k < n && i < rec_cap;
+        u32 pos = 0, re = 0;
+        const u8 *p = buf;
+        if (on) {
+            u32 rel = rec[k];
+            u64 r = ms + rel;
+            p = buf + r;
+            u32 bs = ld_u32le(p);
+            u32 name_len = p[12];
+            u32 n_cigar = ld_u16le(p + 16);
+            u32 l_seq = ld_u32le(p + 20);
+            c.ref_id[i] = (int)ld_u32le(p + 4);
+            c.pos[i] = (int)ld_u32le(p + 8);
+            c.name_len[i] = (u8)name_len;
+            c.mapq[i] = p[13];
+            c.bin[i] = (u16)ld_u16le(p + 14);
+            c.n_cigar[i] = (u16)n_cigar;
+            c.flags[i] = (u16)ld_u16le(p + 18);
+            c.seq_len[i] = l_seq;
+            c.mate_ref_id[i] = (int)ld_u32le(p + 24);
+            c.mate_pos[i] = (int)ld_u32le(p + 28);
+            c.tlen[i] = (int)ld_u32le(p + 32);
+            c.record_offsets[i] = r;
+            c.virtual_offset[i] = vbase | rel;
+            u32 cs = 36u + name_len;
+            u32 ss = cs + 4u * n_cigar;
+            u32 qs = ss + (l_seq + 1u) / 2u;
+            u32 as = qs + l_seq;
+            re = 4u + bs;
+            pos = as;
+            c.cigar_start[i] = cs;
+            c.sequence_start[i] = ss;
+            c.quality_start[i] = qs;
+            c.aux_start[i] = as;
+            c.record_end[i] = re;
         }
-        c.aux_count[i] = nt;
-        c.aux_status[i] = (u8)st;
+        // the fields of the warp's records side by side
+        u32 nt = 0, st = 0;
+        bool walk = on && pos < re;
+        while (__any_sync(FRT_FULL_MASK, walk)) {
+            u32 w0, vo, cn;
+            const u32 nx = aux_field(walk, p, pos, re, &w0, &vo, &cn);
+            if (walk) {
+                if (nx) {
+                    ++nt;
+                    pos = nx;
+                } else {
+                    st = 1;
+                }
+                walk = nx && pos < re;
+            }
+        }
+        if (on) {
+            c.aux_count[i] = nt;
+            c.aux_status[i] = (u8)st;
+        }
     }
 }
 
@@ -688,18 +754,20 @@ __global__ void k_bam_aux_dir(const u8 *buf, const u64 *record_offsets, const u3
 {
     u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (n_dev && *n_dev < n) n = *n_dev;
-    if (i >= n) return;
-    if ((u64)aux_first[i] + aux_count[i] > aux_cap) return;
-    const u8 *p = buf + record_offsets[i];
-    u32 pos = aux_start[i], re = record_end[i], nt = aux_count[i];
-    u32 *out = entries + 3ull * aux_first[i];
-    for (u32 t = 0; t < nt; ++t) {
+    const bool on = i < n && (u64)aux_first[i] + aux_count[i] <= aux_cap;
+    const u8 *p = on ? buf + record_offsets[i] : buf;
+    u32 pos = on ? aux_start[i] : 0u;
+    const u32 re = on ? record_end[i] : 0u, nt = on ? aux_count[i] : 0u;
+    u32 *out = entries + 3ull * (on ? aux_first[i] : 0u);
+    for (u32 t = 0; __any_sync(FRT_FULL_MASK, t < nt); ++t) {
         u32 w0, vo, cn;
-        u32 nx = aux_field(p, pos, re, &w0, &vo, &cn);
-        out[3 * t] = w0;
-        out[3 * t + 1] = vo;
-        out[3 * t + 2] = cn;
-        pos = nx;
+        const u32 nx = aux_field(t < nt, p, pos, re, &w0, &vo, &cn);
+        if (t < nt) {
+            out[3 * t] = w0;
+            out[3 * t + 1] = vo;
+            out[3 * t + 2] = cn;
+            pos = nx;
+        }
     }
 }
 
