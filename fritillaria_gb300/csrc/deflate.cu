@@ -163,21 +163,22 @@ enum PassMode { EMIT_FIXED = 1, EMIT_DYNAMIC = 2 };
 // the lengths past maxlen folded in by the Kraft sum (each excess leaf moves
 // one shorter code a level down), and the shortest codes to the most frequent
 // symbols.  Scratch: keys[512], wt[1024], parent[1024] (u16).
-__device__ void huff_lengths(u32 *freq, u32 n, u32 maxlen, u8 *lens, u32 *keys, u32 *wt, u16 *parent, u32 lane)
+__device__ __forceinline__ void huff_lengths(u32 *freq, u32 n, u32 maxlen, u8 *lens, u32 *keys, u32 *wt, u16 *parent, u32 lane)
 {
-    if (lane == 0) {
-        u32 used = 0;
-        for (u32 s = 0; s < n; ++s) used += freq[s] ? 1u : 0u;
+    u32 used = 0;
+    for (u32 b = 0; b < n; b += 32u) used += __popc(__ballot_sync(FRT_FULL_MASK, b + lane < n && freq[b + lane]));
+    const u32 m = max(used, 2u);
+    if (lane == 0)
         for (u32 s = 0; s < n && used < 2u; ++s)
             if (!freq[s]) freq[s] = 1u, ++used;
-    }
     __syncwarp();
-    for (u32 i = lane; i < 512u; i += 32u) keys[i] = i < n && freq[i] ? (freq[i] << 9) | i : 0xffffffffu;
+    const u32 most = n <= 32u ? 32u : 512u; // keys sorted
+    for (u32 i = lane; i < most; i += 32u) keys[i] = i < n && freq[i] ? (freq[i] << 9) | i : 0xffffffffu;
     for (u32 i = lane; i < n; i += 32u) lens[i] = 0;
     __syncwarp();
-    for (u32 size = 2; size <= 512u; size <<= 1)
+    for (u32 size = 2; size <= most; size <<= 1)
         for (u32 stride = size >> 1; stride; stride >>= 1) {
-            for (u32 t = lane; t < 256u; t += 32u) {
+            for (u32 t = lane; t < most / 2u; t += 32u) {
                 const u32 i = 2u * t - (t & (stride - 1u)), j = i + stride;
                 const bool up = (i & size) == 0;
                 const u32 a = keys[i], b = keys[j];
@@ -185,58 +186,96 @@ __device__ void huff_lengths(u32 *freq, u32 n, u32 maxlen, u8 *lens, u32 *keys, 
             }
             __syncwarp();
         }
+    for (u32 i = lane; i < m; i += 32u) wt[i] = keys[i] >> 9;
+    __syncwarp();
     if (lane == 0) {
-        u32 m = 0;
-        while (m < 512u && keys[m] != 0xffffffffu) ++m;
-        for (u32 i = 0; i < m; ++i) wt[i] = keys[i] >> 9;
-        u32 li = 0, ii = m, nxt = m;
-        while (nxt < 2u * m - 1u) {
-            u32 pick[2];
+        // two queues, the leaves and the inner nodes, their heads in registers
+        constexpr u32 NONE = 0xffffffffu;
+        u32 li = 0, ii = m, leaf = wt[0], inner = NONE;
+        for (u32 nxt = m; nxt < 2u * m - 1u; ++nxt) {
+            u32 sum = 0;
+#pragma unroll
             for (int t = 0; t < 2; ++t) {
-                if (li < m && (ii >= nxt || wt[li] <= wt[ii])) pick[t] = li++;
-                else pick[t] = ii++;
-            }
-            wt[nxt] = wt[pick[0]] + wt[pick[1]];
-            parent[pick[0]] = parent[pick[1]] = (u16)nxt;
-            ++nxt;
-        }
-        // depths, root first; wt[] now holds them
-        wt[2u * m - 2u] = 0;
-        for (int i = (int)(2u * m) - 3; i >= 0; --i) wt[i] = wt[parent[i]] + 1u;
-        u32 cnt[16] = {};
-        for (u32 i = 0; i < m; ++i) ++cnt[min(wt[i], maxlen)];
-        u32 total = 0;
-        for (u32 L = 1; L <= maxlen; ++L) total += cnt[L] << (maxlen - L);
-        while (total > (1u << maxlen)) {
-            --cnt[maxlen];
-            for (u32 L = maxlen - 1u; L > 0; --L)
-                if (cnt[L]) {
-                    --cnt[L];
-                    cnt[L + 1u] += 2u;
-                    break;
+                if (leaf != NONE && leaf <= inner) {
+                    sum += leaf;
+                    parent[li++] = (u16)nxt;
+                    leaf = li < m ? wt[li] : NONE;
+                } else {
+                    sum += inner;
+                    parent[ii++] = (u16)nxt;
+                    inner = ii < nxt ? wt[ii] : NONE;
                 }
-            --total;
+            }
+            wt[nxt] = sum;
+            if (inner == NONE) inner = wt[ii]; // the node just made heads the empty queue
         }
-        u32 k = m; // keys[m - 1] is the most frequent
-        for (u32 L = 1; L <= maxlen; ++L)
-            for (u32 c = 0; c < cnt[L]; ++c) lens[keys[--k] & 511u] = (u8)L;
+    }
+    __syncwarp();
+    // depths: each leaf counts the links to the root; lane L has the leaves at L
+    const u32 root = 2u * m - 2u;
+    u32 cnt = 0;
+    for (u32 b = 0; b < m; b += 32u) {
+        const u32 i = b + lane;
+        u32 d = 0;
+        if (i < m)
+            for (u32 at = i; at != root; at = parent[at]) ++d;
+        d = min(d, maxlen);
+        for (u32 L = 1; L <= maxlen; ++L) {
+            const u32 here = __popc(__ballot_sync(FRT_FULL_MASK, i < m && d == L));
+            if (lane == L) cnt += here;
+        }
+    }
+    u32 total = __reduce_add_sync(FRT_FULL_MASK, lane >= 1u && lane <= maxlen ? cnt << (maxlen - lane) : 0u);
+    while (total > (1u << maxlen)) { // one leaf of the deepest level goes beside one moved a level down
+        const u32 over = __ballot_sync(FRT_FULL_MASK, lane >= 1u && lane < maxlen && cnt) , L = 31u - __clz(over);
+        if (lane == maxlen) --cnt;
+        if (lane == L) --cnt;
+        if (lane == L + 1u) cnt += 2u;
+        --total;
+    }
+    // the shortest codes to the most frequent symbols (keys[m - 1] the most)
+    u32 upto = lane >= 1u && lane <= maxlen ? cnt : 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const u32 y = __shfl_up_sync(FRT_FULL_MASK, upto, d);
+        if (lane >= (u32)d) upto += y;
+    }
+    for (u32 b = 0; b < m; b += 32u) {
+        const u32 i = b + lane;
+        u32 L = 1;
+        for (u32 l = 1; l < maxlen; ++l) L += i >= __shfl_sync(FRT_FULL_MASK, upto, l) ? 1u : 0u;
+        if (i < m) lens[keys[m - 1u - i] & 511u] = (u8)L;
     }
     __syncwarp();
 }
 
 // Canonical codes of lens[0, n) (RFC 1951 3.2.2), reversed for packing.
-__device__ void canonical(const u8 *lens, u32 n, u16 *codes)
+// By a warp: lane L keeps the next code of length L.
+__device__ __forceinline__ void canonical(const u8 *lens, u32 n, u16 *codes, u32 lane)
 {
-    u32 bl[16] = {}, next[16];
-    for (u32 s = 0; s < n; ++s) ++bl[lens[s]];
-    bl[0] = 0;
-    u32 code = 0;
-    for (u32 b = 1; b < 16; ++b) {
-        code = (code + bl[b - 1]) << 1;
-        next[b] = code;
+    u32 cnt = 0;
+    for (u32 b = 0; b < n; b += 32u) {
+        const u32 l = b + lane < n ? lens[b + lane] : 0u;
+        for (u32 L = 1; L < 16u; ++L) {
+            const u32 here = __popc(__ballot_sync(FRT_FULL_MASK, l == L));
+            if (lane == L) cnt += here;
+        }
     }
-    for (u32 s = 0; s < n; ++s)
-        if (lens[s]) codes[s] = (u16)rev(next[lens[s]]++, lens[s]);
+    u32 next = 0, code = 0;
+    for (u32 L = 1; L < 16u; ++L) {
+        code = (code + __shfl_sync(FRT_FULL_MASK, cnt, L - 1u)) << 1;
+        if (lane == L) next = code;
+    }
+    for (u32 b = 0; b < n; b += 32u) {
+        const u32 l = b + lane < n ? lens[b + lane] : 0u;
+        for (u32 L = 1; L < 16u; ++L) {
+            const u32 here = __ballot_sync(FRT_FULL_MASK, l == L);
+            const u32 base = __shfl_sync(FRT_FULL_MASK, next, L);
+            if (l == L) codes[b + lane] = (u16)rev(base + __popc(here & lanemask_lt()), L);
+            if (lane == L) next += __popc(here);
+        }
+    }
+    __syncwarp();
 }
 
 __device__ const u8 kClOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
@@ -247,7 +286,7 @@ __device__ __forceinline__ u32 cl_extra(u32 sym) { return sym == 16 ? 2u : sym =
 // The dynamic trees from the counts (lf[256] counts the end of block), and
 // whether they beat the fixed codes, their header included (the extra bits
 // of lengths and distances are the same either way).
-__device__ void build_trees(WarpState *ws, u32 lane)
+__device__ __forceinline__ void build_trees(WarpState *ws, u32 lane)
 {
     u32 *keys = ws->table, *wt = ws->table + 512;
     u16 *parent = (u16 *)(ws->table + 1536);
@@ -298,27 +337,30 @@ __device__ void build_trees(WarpState *ws, u32 lane)
     }
     __syncwarp();
     huff_lengths(ws->cf, 19, 7, ws->clen, keys, wt, parent, lane);
+    canonical(ws->llen, 286, ws->lcode, lane);
+    canonical(ws->dlen, 30, ws->dcode, lane);
+    canonical(ws->clen, 19, ws->ccode, lane);
+    // bits of the two forms; sums of at most 65,505 symbols' bits fit 32 bits
+    u32 dyn = 0, fix = 0;
+    for (u32 t = lane; t < ws->n_items; t += 32u) {
+        const u32 sym = ws->items[t] & 31u;
+        dyn += ws->clen[sym] + cl_extra(sym);
+    }
+    for (u32 sy = lane; sy < 286; sy += 32u) {
+        dyn += ws->lf[sy] * ws->llen[sy];
+        fix += ws->lf[sy] * fixed_len(sy);
+    }
+    if (lane < 30u) {
+        dyn += ws->df[lane] * ws->dlen[lane];
+        fix += ws->df[lane] * 5u;
+    }
+    dyn = __reduce_add_sync(FRT_FULL_MASK, dyn);
+    fix = __reduce_add_sync(FRT_FULL_MASK, fix);
     if (lane == 0) {
         u32 hclen = 19;
         while (hclen > 4 && !ws->clen[kClOrder[hclen - 1]]) --hclen;
         ws->hclen = hclen;
-        canonical(ws->llen, 286, ws->lcode);
-        canonical(ws->dlen, 30, ws->dcode);
-        canonical(ws->clen, 19, ws->ccode);
-        u64 dyn = 17u + 3u * hclen, fix = 3;
-        for (u32 t = 0; t < ws->n_items; ++t) {
-            const u32 sym = ws->items[t] & 31u;
-            dyn += ws->clen[sym] + cl_extra(sym);
-        }
-        for (u32 sy = 0; sy < 286; ++sy) {
-            dyn += (u64)ws->lf[sy] * ws->llen[sy];
-            fix += (u64)ws->lf[sy] * fixed_len(sy);
-        }
-        for (u32 d = 0; d < 30; ++d) {
-            dyn += (u64)ws->df[d] * ws->dlen[d];
-            fix += (u64)ws->df[d] * 5u;
-        }
-        ws->dynamic = dyn < fix ? 1u : 0u;
+        ws->dynamic = dyn + 17u + 3u * hclen < fix + 3u ? 1u : 0u;
     }
     __syncwarp();
 }
@@ -331,8 +373,10 @@ __device__ __forceinline__ void flush_some(WarpState *ws, u32 *slot, u32 bitpos,
     }
 }
 
-constexpr u32 kThreads = 512, kWarps = kThreads / 32;
+constexpr u32 kThreads = 1024, kWarps = kThreads / 32; // parts of a parse: 16 of them took half as long again
+constexpr u32 kLinkWarps = 16; // their tables fill the room of `match`
 constexpr u32 kWarm = 512; // bytes a warp parses before its part
+constexpr u32 kOthers = 40;
 
 // A chunk's state: all of an SM's shared memory.
 struct ChunkState {
@@ -340,11 +384,12 @@ struct ChunkState {
     u16 prev[65536];
     union {
         u8 match[65536];                  // match length with it, less 2, 255 for 257 and 258; 0: no match
-        u16 last[kWarps][1u << kHashBits]; // while prev is built: each warp's last position + 1 of a hash
+        u16 last[kLinkWarps][1u << kHashBits]; // while prev is built: each warp's last position + 1 of a hash
     };
     u32 inside[2048]; // positions inside a match, but its first
     u32 first[2048];  // first positions of matches
     u32 start[kWarps], end[kWarps], sums[kWarps];
+    u32 other[kWarps][kOthers]; // a warp's matches with a candidate that is not prev: position | candidate << 16
     WarpState tree;
 };
 
@@ -381,28 +426,37 @@ __device__ __forceinline__ u32 match_length(const u8 *p, u32 q, u32 c, u32 len)
 // with a table of its own (lanes of one hash find each other by match_any);
 // then each hash's last position before every part, and the positions their
 // part had no earlier one for.
-__device__ void link_prefixes(ChunkState *cs, const u8 *p, u32 len)
+__device__ __forceinline__ void link_prefixes(ChunkState *cs, const u8 *p, u32 len)
 {
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
-    const u32 part = (len + kThreads - 1) / kThreads * 32u;
-    u16 *last = cs->last[warp];
-    for (u32 i = tid; i < (u32)kWarps << (kHashBits - 1); i += kThreads) ((u32 *)cs->last)[i] = 0;
+    const u32 part = (len + 32u * kLinkWarps - 1) / (32u * kLinkWarps) * 32u;
+    u16 *last = cs->last[warp % kLinkWarps];
+    for (u32 i = tid; i < kLinkWarps << (kHashBits - 1); i += kThreads) ((u32 *)cs->last)[i] = 0;
     __syncthreads();
-    const u32 to = min(len, (warp + 1) * part);
+    const u32 to = warp < kLinkWarps ? min(len, (warp + 1) * part) : 0u;
     for (u32 b = warp * part; b < to; b += 32) {
         const u32 q = b + lane;
         const bool in = q < to && q + 3u <= len;
         const u32 h = in ? hash_at(p, q) : 0u;
-        const u32 peers = __match_any_sync(FRT_FULL_MASK, in ? h : 0x10000u + lane), below = peers & lanemask_lt();
-        if (q < to) cs->prev[q] = !in ? 0u : (u16)(below ? b + 32u - __clz(below) : last[h]);
+        u32 before = in ? last[h] : 0u;
         __syncwarp();
-        if (in && (peers >> lane) == 1u) last[h] = (u16)(q + 1u);
+        if (in) last[h] = (u16)(q + 1u);
+        __syncwarp();
+        // lanes of one hash: one of them has written (seen without match_any,
+        // whose 32 distinct values cost more than the rest of the turn)
+        if (__any_sync(FRT_FULL_MASK, in && last[h] != (u16)(q + 1u))) {
+            const u32 peers = __match_any_sync(FRT_FULL_MASK, in ? h : 0x10000u + lane), below = peers & lanemask_lt();
+            if (below) before = b + 32u - __clz(below);
+            __syncwarp();
+            if (in && (peers >> lane) == 1u) last[h] = (u16)(q + 1u);
+        }
+        if (q < to) cs->prev[q] = (u16)(in ? before : 0u);
         __syncwarp();
     }
     __syncthreads();
     for (u32 h = tid; h < (1u << kHashBits); h += kThreads) {
         u16 run = 0;
-        for (u32 w = 0; w < kWarps; ++w) {
+        for (u32 w = 0; w < kLinkWarps; ++w) {
             const u16 t = cs->last[w][h];
             cs->last[w][h] = run;
             if (t) run = t;
@@ -417,10 +471,10 @@ __device__ void link_prefixes(ChunkState *cs, const u8 *p, u32 len)
 // One step of the greedy parse at `pos`, by a warp (uniform result): the first
 // of the next 32 positions that matches the latest position before `pos` with
 // its hash ends a run of literals.  Returns where the step ends; `m`, `L` and
-// `c` are its match (L 0: none).  It depends on `pos` alone, so parts of the
+// `c` are its match (L 0: none), `again` whether c is not prev.  It depends on `pos` alone, so parts of the
 // chunk can be parsed apart.  That candidate is prev, or, where prev lies in
 // the step itself, further back along prev (rare: looked at by its bytes).
-__device__ __forceinline__ u32 parse_step(const ChunkState *cs, const u8 *p, u32 len, u32 pos, u32 &m, u32 &L, u32 &c)
+__device__ __forceinline__ u32 parse_step(const ChunkState *cs, const u8 *p, u32 len, u32 pos, u32 &m, u32 &L, u32 &c, bool &again)
 {
     const u32 lane = lane_id(), q = pos + lane;
     const bool in = q + 3u <= len;
@@ -429,7 +483,7 @@ __device__ __forceinline__ u32 parse_step(const ChunkState *cs, const u8 *p, u32
     u32 k = hits ? (u32)__ffs(hits) - 1u : 32u;
     const u32 late = __ballot_sync(FRT_FULL_MASK, pv > pos) & (k < 32u ? (1u << k) - 1u : 0xffffffffu);
     u32 at = pv;
-    bool again = false;
+    again = false;
     if (late) {
         const bool mine = (late >> lane) & 1u;
         while (__any_sync(FRT_FULL_MASK, mine && at > pos))
@@ -454,45 +508,80 @@ __device__ __forceinline__ u32 parse_step(const ChunkState *cs, const u8 *p, u32
     return m + L;
 }
 
-// The parse of the chunk: its matches marked in `first` and `inside`, with
-// prev and match their candidates and lengths.  Each warp parses a part from
-// where a parse begun kWarm bytes before it first reaches it; where the part
-// before ends elsewhere it goes again from there.
-__device__ void parse(ChunkState *cs, const u8 *p, u32 len)
+// Marks the match of L bytes at m in `first` and `inside`, by a warp.
+__device__ __forceinline__ void mark_match(ChunkState *cs, u32 m, u32 L)
 {
-    const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
+    // lane 31 marks the first byte, the others the words of [m + 1, m + L): at
+    // most 10, most often one
+    const u32 lane = lane_id(), a = m + 1u, e = m + L, w = lane == 31u ? m >> 5 : (a >> 5) + lane;
+    const u32 lo = max(a, 32u * w) & 31u, hi = min(e - 32u * w, 32u);
+    const u32 bits = lane == 31u ? 1u << (m & 31u) : (0xffffffffu << lo) & (hi == 32u ? 0xffffffffu : (1u << (hi & 31u)) - 1u);
+    if (lane == 31u || 32u * w < e) atomicOr((lane == 31u ? cs->first : cs->inside) + w, bits);
+}
+
+__device__ __forceinline__ void clear_marks(ChunkState *cs)
+{
+    for (u32 i = threadIdx.x; i < 2048u; i += kThreads) cs->inside[i] = cs->first[i] = 0;
+    __syncthreads();
+}
+
+// The parse of the chunk: its matches marked in `first` and `inside`, with
+// prev and match their candidates and lengths.  Each warp parses and marks a
+// part from where a parse begun kWarm bytes before it first reaches it.  Where
+// a part then does not start where the one before ended (rare), the marks go,
+// the starts are found, each such part again from its right place, and all
+// parts are marked anew.
+__device__ __forceinline__ void parse(ChunkState *cs, const u8 *p, u32 len)
+{
+    const u32 lane = threadIdx.x & 31u, warp = threadIdx.x / 32;
     const u32 part = (len + kWarps - 1) / kWarps, from = min(len, warp * part), to = min(len, from + part);
-    u32 m, L, c, pos = from > kWarm ? from - kWarm : 0u;
-    while (pos < from) pos = parse_step(cs, p, len, pos, m, L, c);
+    bool again;
+    u32 m, L, c, pos = from > kWarm ? from - kWarm : 0u, others = 0;
+    clear_marks(cs);
+    while (pos < from) pos = parse_step(cs, p, len, pos, m, L, c, again);
     u32 start = pos;
-    bool go = true;
+    while (pos < to) {
+        pos = parse_step(cs, p, len, pos, m, L, c, again);
+        if (L) {
+            mark_match(cs, m, L);
+            if (again) { // prev stays as it is until the parse is proven
+                if (lane == 0 && others < kOthers) cs->other[warp][others] = m | (c << 16);
+                ++others;
+            }
+        }
+    }
+    if (lane == 0) cs->end[warp] = pos;
+    __syncthreads();
+    if (!__syncthreads_or(start != (warp ? cs->end[warp - 1] : 0u) || others > kOthers)) {
+        for (u32 i = lane; i < others; i += 32u) {
+            const u32 q = cs->other[warp][i] & 0xffffu, at = cs->other[warp][i] >> 16;
+            cs->prev[q] = (u16)(at + 1u);
+            cs->match[q] = (u8)min(match_length(p, q, at, len) - 2u, 255u);
+        }
+        __syncthreads();
+        return;
+    }
     while (true) {
+        const u32 before = warp ? cs->end[warp - 1] : 0u;
+        const bool go = start != before;
+        start = before;
+        if (!__syncthreads_or(go)) break;
         if (go) {
             pos = start;
-            while (pos < to) pos = parse_step(cs, p, len, pos, m, L, c);
+            while (pos < to) pos = parse_step(cs, p, len, pos, m, L, c, again);
             if (lane == 0) cs->end[warp] = pos;
         }
         __syncthreads();
-        const u32 before = warp ? cs->end[warp - 1] : 0u;
-        go = start != before;
-        start = before;
-        if (!__syncthreads_or(go)) break;
     }
-    for (u32 i = tid; i < 2048u; i += kThreads) cs->inside[i] = cs->first[i] = 0;
-    __syncthreads();
+    clear_marks(cs);
     for (pos = start; pos < to;) {
-        pos = parse_step(cs, p, len, pos, m, L, c);
+        pos = parse_step(cs, p, len, pos, m, L, c, again);
         if (L) {
             if (lane == 0) {
                 cs->prev[m] = (u16)(c + 1u);
                 cs->match[m] = (u8)min(L - 2u, 255u);
-                atomicOr(&cs->first[m >> 5], 1u << (m & 31u));
             }
-            const u32 a = m + 1u, e = m + L, w = (a >> 5) + lane; // [a, e): at most 10 words
-            if (32u * w < e) {
-                const u32 lo = max(a, 32u * w) & 31u, hi = min(e - 32u * w, 32u);
-                atomicOr(&cs->inside[w], (0xffffffffu << lo) & (hi == 32u ? 0xffffffffu : (1u << hi) - 1u));
-            }
+            mark_match(cs, m, L);
             __syncwarp();
         }
     }
@@ -510,16 +599,17 @@ __device__ __forceinline__ void match_symbols(const ChunkState *cs, const u8 *p,
     dist_sym(q - c, &ds, &dex, &dnb);
 }
 
-// The symbol at position q: its code and extra bits (at most 20, a distance's
-// 28 after them) and their lengths.
+// A symbol's code and extra bits (at most 20, a distance's 28 after them) and
+// their lengths: the match that starts at q, or the literal `byte`.
 template <int MODE>
-__device__ __forceinline__ void symbol_bits(const ChunkState *cs, const u8 *p, u32 len, u32 q, u32 &v, u32 &nb, u32 &v2, u32 &nb2)
+__device__ __forceinline__ void symbol_bits(const ChunkState *cs, const u8 *p, u32 len, u32 q, bool match, u32 byte, u32 &v, u32 &nb,
+                                            u32 &v2, u32 &nb2)
 {
     const WarpState *ws = &cs->tree;
     nb2 = 0;
-    if (!((cs->first[q >> 5] >> (q & 31u)) & 1u)) {
-        if (MODE == EMIT_FIXED) fixed_lit(p[q], &v, &nb);
-        else v = ws->lcode[p[q]], nb = ws->llen[p[q]];
+    if (!match) {
+        if (MODE == EMIT_FIXED) fixed_lit(byte, &v, &nb);
+        else v = ws->lcode[byte], nb = ws->llen[byte];
         return;
     }
     u32 ls, lex, lnb, ds, dex, dnb;
@@ -564,20 +654,42 @@ struct BitRun {
     }
 };
 
+// Calls f(v, nb, v2, nb2) for each symbol of positions [from, to), in order;
+// `from` is a multiple of 32.
+template <int MODE, class F>
+__device__ __forceinline__ void each_symbol(const ChunkState *cs, const u8 *p, u32 len, u32 from, u32 to, F f)
+{
+    for (u32 b = from; b < to; b += 32) {
+        u32 m = ~cs->inside[b >> 5];
+        if (to - b < 32u) m &= (1u << (to - b)) - 1u;
+        const u32 first = cs->first[b >> 5];
+        u32 at = 0xffffffffu, four = 0;
+        for (; m; m &= m - 1) {
+            const u32 k = (u32)__ffs(m) - 1u, q = b + k;
+            if ((k >> 2) != at && !((first >> k) & 1u)) {
+                at = k >> 2;
+                if (b + 4u * at + 4u <= len) four = load4(p, b + 4u * at);
+                else
+                    for (u32 i = four = 0; b + 4u * at + i < len; ++i) four |= (u32)p[b + 4u * at + i] << (8u * i);
+            }
+            u32 v, nb, v2, nb2;
+            symbol_bits<MODE>(cs, p, len, q, (first >> k) & 1u, (four >> (8u * (k & 3u))) & 0xffu, v, nb, v2, nb2);
+            f(v, nb, v2, nb2);
+        }
+    }
+}
+
 // The chunk's symbols as bits from `bit` on in the slot: each thread takes a
 // run of positions, its place from a sum over the team.  Returns the bit past
 // the last, the same in every thread, or 0 where the block with its
 // end-of-block code of `eob` bits would outgrow a BGZF block.
-template <int MODE> __device__ u32 emit(ChunkState *cs, const u8 *p, u32 len, u32 *slot, u32 bit, u32 eob)
+template <int MODE> __device__ __forceinline__ u32 emit(ChunkState *cs, const u8 *p, u32 len, u32 *slot, u32 bit, u32 eob)
 {
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
-    const u32 per = (len + kThreads - 1) / kThreads, from = min(len, tid * per), to = min(len, from + per);
-    u32 v, nb, v2, nb2, sum = 0;
-    for (u32 q = from; q < to; ++q)
-        if (!((cs->inside[q >> 5] >> (q & 31u)) & 1u)) {
-            symbol_bits<MODE>(cs, p, len, q, v, nb, v2, nb2);
-            sum += nb + nb2;
-        }
+    // whole words of marks a thread; the chunk's bytes four at a time
+    const u32 per = (len + 32u * kThreads - 1) / (32u * kThreads) * 32u, from = min(len, tid * per), to = min(len, from + per);
+    u32 sum = 0;
+    each_symbol<MODE>(cs, p, len, from, to, [&](u32, u32 nb, u32, u32 nb2) { sum += nb + nb2; });
     u32 x = sum;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -596,12 +708,10 @@ template <int MODE> __device__ u32 emit(ChunkState *cs, const u8 *p, u32 len, u3
     for (u32 w = ((bit + 31u) >> 5) + tid; w < clear; w += kThreads) slot[w] = 0;
     __syncthreads();
     BitRun run(slot, before + x - sum);
-    for (u32 q = from; q < to; ++q)
-        if (!((cs->inside[q >> 5] >> (q & 31u)) & 1u)) {
-            symbol_bits<MODE>(cs, p, len, q, v, nb, v2, nb2);
-            run.put(v, nb);
-            if (nb2) run.put(v2, nb2);
-        }
+    each_symbol<MODE>(cs, p, len, from, to, [&](u32 v, u32 nb, u32 v2, u32 nb2) {
+        run.put(v, nb);
+        if (nb2) run.put(v2, nb2);
+    });
     run.done();
     return total;
 }
@@ -613,11 +723,11 @@ template <int MODE> __device__ u32 emit(ChunkState *cs, const u8 *p, u32 len, u3
 // whatever the number of chunks.  What a step does depends only on where it
 // starts, once every position's earlier positions of its hash are linked: so
 // the links and every position's match length are made by all threads at once,
-// sixteen warps parse sixteen parts (parses from different starts fall into
+// thirty-two warps parse as many parts (parses from different starts fall into
 // step within a few matches), and counts and codes are taken position by
 // position.  The stream is bit for bit the one-warp form's.  Measured on GB300
 // through compress_batch_device: 454 chunks of short reads (29.6 MB) 19.8 ->
-// 3.06 ms.
+// 1.72 ms.
 __global__ void __launch_bounds__(kThreads) k_deflate_chunks(const u8 *data, const u64 *bounds, u32 n, u8 *slots,
                                                              u32 *deflate_len, u32 *crcs)
 {
@@ -628,17 +738,33 @@ __global__ void __launch_bounds__(kThreads) k_deflate_chunks(const u8 *data, con
     const u8 *p = data + bounds[chunk];
     const u32 len = (u32)(bounds[chunk + 1] - bounds[chunk]);
 
-    // CRC-32: thread slices from zero, shifted past the bytes after them
+    // CRC-32: thread slices of whole words from zero, shifted past the bytes
+    // after them; the byte table in the tree builder's scratch
     {
-        const u32 s = (len + kThreads - 1) / kThreads, b0 = min(len, tid * s), b1 = min(len, b0 + s);
-        u32 c = tid == 0 ? 0xffffffffu : 0u;
-        for (u32 i = b0; i < b1; ++i) c = g_bcrc.t[(c ^ p[i]) & 0xffu] ^ (c >> 8);
-        if (c) c = crc_shift(c, len - b1);
+        u32 *t = ws->table;
+        for (u32 i = tid; i < 256u; i += kThreads) t[i] = g_bcrc.t[i];
+        __syncthreads();
+        const u32 head = min(len, (4u - (u32)((u64)p & 3u)) & 3u), words = (len - head) / 4u;
+        const u32 per = (words + kThreads - 1) / kThreads, w0 = min(words, tid * per), w1 = min(words, w0 + per);
+        const u32 *w = (const u32 *)(p + head);
+        u32 c = 0, end = head + 4u * w1;
+        if (tid == 0) {
+            c = 0xffffffffu;
+            for (u32 i = 0; i < head; ++i) c = t[(c ^ p[i]) & 0xffu] ^ (c >> 8);
+        }
+        for (u32 i = w0; i < w1; ++i) {
+            c ^= __ldg(w + i);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) c = t[c & 0xffu] ^ (c >> 8);
+        }
+        if (w1 == words && (w0 < words || tid == 0))
+            for (; end < len; ++end) c = t[(c ^ p[end]) & 0xffu] ^ (c >> 8);
+        if (c) c = crc_shift(c, len - end);
         c = __reduce_xor_sync(FRT_FULL_MASK, c);
         if (lane == 0) cs->sums[warp] = c;
         __syncthreads();
         if (tid == 0) {
-            for (u32 w = 1; w < kWarps; ++w) c ^= cs->sums[w];
+            for (u32 k = 1; k < kWarps; ++k) c ^= cs->sums[k];
             crcs[chunk] = ~c;
         }
         __syncthreads();

@@ -1,6 +1,6 @@
 """The device deflate at the sizes where its parts meet: chunks around a step (32
 positions), a thread's and a warp's share, the window, the largest payload, and
-chunks whose length leaves some of the sixteen parsing warps nothing; runs,
+chunks whose length leaves some of the parsing warps nothing; runs,
 matches across parts, long matches and noise.  zlib turns every block back into
 its chunk, and the same chunk gives the same block alone and among others."""
 
