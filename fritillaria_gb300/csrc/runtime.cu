@@ -126,26 +126,63 @@ struct DeviceGuard {
     }
 };
 
-// Host bytes in page-locked memory, so H2D copies run at full link speed.
+PinnedPool::~PinnedPool()
+{
+    for (const Buffer &b : kept) cudaFreeHost(b.p);
+}
+
+uint8_t *PinnedPool::take(size_t want, size_t *cap)
+{
+    std::lock_guard<std::mutex> lk(mu);
+    size_t best = kept.size();
+    for (size_t i = 0; i < kept.size(); ++i)
+        if (kept[i].cap >= want && (best == kept.size() || kept[i].cap < kept[best].cap)) best = i;
+    if (best == kept.size()) return nullptr;
+    uint8_t *p = kept[best].p;
+    *cap = kept[best].cap;
+    kept.erase(kept.begin() + (ptrdiff_t)best);
+    return p;
+}
+
+void PinnedPool::give(uint8_t *p, size_t cap)
+{
+    if (!p) return;
+    if (cap <= MAX_BYTES) {
+        std::lock_guard<std::mutex> lk(mu);
+        if (kept.size() < MAX_BUFFERS) {
+            kept.push_back({p, cap});
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+// Host bytes in page-locked memory, so H2D copies run at full link speed; from
+// the codec's pool, and back to it where no copy can still be reading them.
 struct PinnedBytes {
+    std::shared_ptr<PinnedPool> pool;
     uint8_t *p = nullptr;
     size_t n = 0, cap = 0;
-    ~PinnedBytes()
+    bool idle = true; // no copy in flight
+    ~PinnedBytes() { drop(); }
+    void drop()
     {
-        if (p) cudaFreeHost(p);
+        if (p && pool && idle) pool->give(p, cap);
+        else if (p) cudaFreeHost(p);
+        p = nullptr;
     }
     bool reserve(size_t want)
     {
         if (want <= cap) return true;
         size_t nc = cap ? cap : 1 << 20;
         while (nc < want) nc *= 2;
-        uint8_t *q = nullptr;
-        if (cudaMallocHost((void **)&q, nc) != cudaSuccess) {
+        uint8_t *q = pool ? pool->take(want, &nc) : nullptr;
+        if (!q && cudaMallocHost((void **)&q, nc) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
         if (n) memcpy(q, p, n);
-        if (p) cudaFreeHost(p);
+        drop();
         p = q;
         cap = nc;
         return true;
@@ -632,6 +669,7 @@ static int reader_new(frt_codec *codec, frt_reader **out, frt_error *err, frt_re
         return FRT_ERR_INVALID_ARGUMENT;
     }
     r->codec = codec;
+    r->compressed.pool = codec->pinned;
     *out = r;
     return FRT_OK;
 }
@@ -750,8 +788,10 @@ extern "C" int frt_reader_next_batch(frt_reader *r, frt_inflate_batch **out, uin
             continue;
         }
         frt_inflate_batch *b = nullptr;
+        r->compressed.idle = false;
         rc = inflate_batch(r->codec, r->compressed.p, r->compressed.n, r->spans.data(), r->spans.size(), &b, err);
         if (rc) return rc;
+        r->compressed.idle = true; // a batch is handed out once its stream is done
         if (b->len == 0) {
             batch_release(b);
             if (r->exhausted) return FRT_OK;
