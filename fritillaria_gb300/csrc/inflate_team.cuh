@@ -43,13 +43,14 @@
 // member's start, whose checks and statuses are the reference's.
 //
 // Measured on GB300 against the serial form (its tuned shape, the inflate alone):
-// 1M short reads 8.7 -> 2.54 ms (117 GB/s of output), ultra-long reads 6.3 ->
-// 1.33 ms, BCF 3.6 -> 0.80 ms, FASTQ 4.6 -> 1.18 ms, FASTA 3.3 -> 0.65 ms; one
-// short-read member alone 4.4 -> 0.145 ms.  The integer ALUs bound it (ncu: 62%
-// of their peak averaged over phases, 24 warps an SM, 441,000 warp instructions
+// 1M short reads 8.7 -> 2.48 ms (119 GB/s of output), ultra-long reads 6.3 ->
+// 1.26 ms, BCF 3.6 -> 0.78 ms, FASTQ 4.6 -> 1.13 ms, FASTA 3.3 -> 0.63 ms; one
+// short-read member alone 4.4 -> 0.139 ms.  The integer ALUs bound it (ncu: 62%
+// of their peak averaged over phases, 24 warps an SM, 440,000 warp instructions
 // a short-read member; DRAM under 3%).  Twelve warps: ten and eleven measured
-// even to 3% slower, sixteen slower (the sync pass grows with the lanes).  Two
-// CTAs fill the shared memory.
+// even to 3% slower, sixteen slower (the sync pass grows with the lanes), and
+// 192 to 320 decoding lanes of the twelve warps' 384 0-10% slower.  Two CTAs
+// fill the shared memory; one alone gives two thirds of the rate.
 #pragma once
 
 namespace team {
@@ -95,7 +96,7 @@ constexpr u32 GROUP_MATCHES = 256 / 3 + 1; // most matches that start in 256 byt
 // member's first byte lies at its HBM address modulo 16.
 template <int NW> struct Smem {
     static constexpr u32 NT = 32 * NW;
-    static constexpr u32 WIN = 512 * NW; // bytes of a copy window
+    static constexpr u32 WIN = 256 * NW; // bytes of a copy window: a group a warp (two measured 2% slower)
     alignas(16) u8 out[OUT_MAX + 16]; // the member's output, at the alignment of its place in HBM
     u32 starts[MARKS];                // first bytes of matches
     u32 tab[TAB];
@@ -464,6 +465,84 @@ __device__ __forceinline__ u32 bits_at(const u32 *stage, u32 a)
     return __funnelshift_r(stage[a >> 5], stage[(a >> 5) + 1], a);
 }
 
+// The n code lengths from staged bit `a` on, into sm->lens, by the team; the
+// code-length code's table is in place, and sm->sh[5] is set to the bits they
+// take.  Returns 1, 0 where the serial form is to take the member, or -1 where
+// they go on past SPAN bits (all uniform).
+template <int NW, u32 SPAN> __device__ __forceinline__ int follow_lengths(Smem<NW> *sm, u32 a, u32 n)
+{
+    constexpr u32 NT = Smem<NW>::NT, PER = (SPAN + NT - 1) / NT;
+    u16 *const jump = (u16 *)sm->tab;
+    const u32 *const clt = sm->val;
+    u16 *const place = (u16 *)(sm->val + 128);
+    u8 *const value = (u8 *)(place + 512);
+    const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
+#pragma unroll
+    for (u32 k = 0; k < PER; ++k) {
+        const u32 p = tid + k * NT;
+        if (p < SPAN) {
+            const u32 e = clt[bits_at(sm->stage, a + p) & 127u];
+            jump[p] = (u16)min(p + (e & 15u) + ((e >> 4) & 15u), SPAN);
+        }
+    }
+    if (tid == 0) {
+        jump[SPAN] = (u16)SPAN;
+        place[0] = 0;
+    }
+    __syncthreads();
+    for (u32 r = 1; r < NT; r <<= 1) {
+        u32 j[PER];
+#pragma unroll
+        for (u32 k = 0; k < PER; ++k) {
+            const u32 p = tid + k * NT;
+            j[k] = p < SPAN ? jump[jump[p]] : 0u;
+        }
+        if (tid < r && tid + r < NT) place[tid + r] = jump[place[tid]];
+        __syncthreads();
+#pragma unroll
+        for (u32 k = 0; k < PER; ++k) {
+            const u32 p = tid + k * NT;
+            if (p < SPAN) jump[p] = (u16)j[k];
+        }
+        __syncthreads();
+    }
+    // thread r holds symbol r: the lengths before it, and for a repeat the
+    // last symbol before it that is none
+    const u32 p = place[tid];
+    const u32 w = p < SPAN ? bits_at(sm->stage, a + p) : 0u, e = clt[w & 127u], sym = e >> 8;
+    const u32 x = (w >> (e & 15u)) & ((1u << ((e >> 4) & 15u)) - 1u);
+    const u32 rep = p >= SPAN ? 0u : (sym < 16 ? 1u : (sym == 18 ? 11u : 3u) + x);
+    value[tid] = (u8)(sym < 16 ? sym : 0u);
+    u32 sum = rep, from = sym != 16 ? tid + 1u : 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const u32 y = __shfl_up_sync(FRT_FULL_MASK, sum, d), z = __shfl_up_sync(FRT_FULL_MASK, from, d);
+        if ((int)lane >= d) {
+            sum += y;
+            from = max(from, z);
+        }
+    }
+    if (lane == 31) {
+        sm->wa[warp] = sum;
+        sm->wb[warp] = from;
+    }
+    __syncthreads();
+    sum += __reduce_add_sync(FRT_FULL_MASK, lane < warp ? sm->wa[lane] : 0u);
+    from = max(from, __reduce_max_sync(FRT_FULL_MASK, lane < warp ? sm->wb[lane] : 0u));
+    const u32 at = sum - rep;
+    bool bad = false;
+    if (rep && at < n) {
+        bad = sum > n || from == 0;
+        if (!bad) {
+            const u8 v = value[from - 1];
+            for (u32 i = at; i < sum; ++i) sm->lens[i] = v;
+            if (sum == n) sm->sh[5] = p + (e & 15u) + ((e >> 4) & 15u);
+        }
+    }
+    if (__syncthreads_or(bad)) return 0;
+    return __syncthreads_or(tid == NT - 1 && sum < n) ? -1 : 1;
+}
+
 // The code lengths of a dynamic block, into sm->lens, by the team.  `a` is the
 // staged bit after the block's three header bits and moves past the lengths.
 //
@@ -475,13 +554,10 @@ __device__ __forceinline__ u32 bits_at(const u32 *stage, u32 a)
 // False (uniform): the serial form is to take the member.
 template <int NW> __device__ __forceinline__ bool read_lengths(Smem<NW> *sm, u32 &a, u32 &nlen, u32 &ndist)
 {
-    constexpr u32 NT = Smem<NW>::NT, PER = (HEAD_BITS + NT - 1) / NT;
+    constexpr u32 NT = Smem<NW>::NT;
     static_assert(NT >= 316, "a thread per symbol");
     static_assert(2 * (HEAD_BITS + 1) <= 4 * EXTRA_AT && 4 * 128 + 2 * 512 + 512 <= 4 * EXTRA_AT, "scratch in the tables' place");
-    u16 *const jump = (u16 *)sm->tab; // the tables are free until the block's are built
-    u32 *const clt = sm->val;
-    u16 *const place = (u16 *)(sm->val + 128);
-    u8 *const value = (u8 *)(place + 512);
+    u32 *const clt = sm->val; // the tables are free until the block's are built
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
     const u32 h = bits_at(sm->stage, a);
     nlen = (h & 31u) + 257;
@@ -510,69 +586,11 @@ template <int NW> __device__ __forceinline__ bool read_lengths(Smem<NW> *sm, u32
                 clt[j] = L | ((lane == 16 ? 2u : (lane == 17 ? 3u : (lane == 18 ? 7u : 0u))) << 4) | (lane << 8);
     }
     a += 3 * ncode;
-    if (tid == 0) place[0] = 0;
     if (__syncthreads_or(bad)) return false;
-#pragma unroll
-    for (u32 k = 0; k < PER; ++k) {
-        const u32 p = tid + k * NT;
-        if (p < HEAD_BITS) {
-            const u32 e = clt[bits_at(sm->stage, a + p) & 127u];
-            jump[p] = (u16)min(p + (e & 15u) + ((e >> 4) & 15u), HEAD_BITS);
-        }
-    }
-    if (tid == 0) jump[HEAD_BITS] = (u16)HEAD_BITS;
-    __syncthreads();
-    for (u32 r = 1; r < NT; r <<= 1) {
-        u32 j[PER];
-#pragma unroll
-        for (u32 k = 0; k < PER; ++k) {
-            const u32 p = tid + k * NT;
-            j[k] = p < HEAD_BITS ? jump[jump[p]] : 0u;
-        }
-        if (tid < r) place[tid + r] = jump[place[tid]];
-        __syncthreads();
-#pragma unroll
-        for (u32 k = 0; k < PER; ++k) {
-            const u32 p = tid + k * NT;
-            if (p < HEAD_BITS) jump[p] = (u16)j[k];
-        }
-        __syncthreads();
-    }
-    // thread r holds symbol r: the lengths before it, and for a repeat the
-    // last symbol before it that is none
-    const u32 p = place[tid];
-    const u32 w = p < HEAD_BITS ? bits_at(sm->stage, a + p) : 0u, e = clt[w & 127u], sym = e >> 8;
-    const u32 x = (w >> (e & 15u)) & ((1u << ((e >> 4) & 15u)) - 1u);
-    const u32 rep = p >= HEAD_BITS ? 0u : (sym < 16 ? 1u : (sym == 18 ? 11u : 3u) + x);
-    value[tid] = (u8)(sym < 16 ? sym : 0u);
-    u32 sum = rep, from = sym != 16 ? tid + 1u : 0u;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const u32 y = __shfl_up_sync(FRT_FULL_MASK, sum, d), z = __shfl_up_sync(FRT_FULL_MASK, from, d);
-        if ((int)lane >= d) {
-            sum += y;
-            from = max(from, z);
-        }
-    }
-    if (lane == 31) {
-        sm->wa[warp] = sum;
-        sm->wb[warp] = from;
-    }
-    __syncthreads();
-    sum += __reduce_add_sync(FRT_FULL_MASK, lane < warp ? sm->wa[lane] : 0u);
-    from = max(from, __reduce_max_sync(FRT_FULL_MASK, lane < warp ? sm->wb[lane] : 0u));
-    const u32 at = sum - rep;
-    bad = false;
-    if (rep && at < n) {
-        bad = sum > n || from == 0;
-        if (!bad) {
-            const u8 v = value[from - 1];
-            for (u32 i = at; i < sum; ++i) sm->lens[i] = v;
-            if (sum == n) sm->sh[5] = p + (e & 15u) + ((e >> 4) & 15u);
-        }
-    }
-    if (tid == NT - 1 && sum < n) bad = true;
-    if (__syncthreads_or(bad)) return false;
+    // half the positions do for most headers (~1,000 bits for short reads)
+    int got = follow_lengths<NW, HEAD_BITS / 2>(sm, a, n);
+    if (got < 0) got = follow_lengths<NW, HEAD_BITS>(sm, a, n);
+    if (got <= 0) return false;
     a += sm->sh[5];
     return sm->lens[256] != 0;
 }
@@ -761,7 +779,7 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
                                              u32 cap, u32 off, u32 &bitpos, u32 &pos, bool last_block)
 {
     constexpr u32 NT = Smem<NW>::NT;
-    constexpr u32 SYNC_BITS = 768, MIN_SEG = 256;
+    constexpr u32 SYNC_BITS = 640, MIN_SEG = 192; // 512 and 768, 256 and 384 measured 0-4% slower
     // a lane runs at most one symbol (48 bits) past its segment and loads up
     // to three words ahead
     constexpr u32 ROUND_BITS = 32u * (STAGE_WORDS - 6);
