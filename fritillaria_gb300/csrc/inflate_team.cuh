@@ -788,6 +788,7 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
     const u32 tab = smem_u32(sm->tab), stage = smem_u32(sm->stage), out = smem_u32(sm->out), starts = smem_u32(sm->starts);
     while (true) {
         const u32 rem = total - bitpos;
+        if (rem == 0) return false; // ends before the block does
         // the last block takes the rest of the payload, others about what the
         // one before took: a block that ends in its round takes one round, and
         // lanes past its end work for nothing

@@ -66,3 +66,32 @@ def test_edges_equal_zlib(gpu, kind):
     got, offs = gpu.CudaCodec(0).inflate_batch(data, spans)
     for i, (_, raw) in enumerate(streams):
         assert got[offs[i]:offs[i + 1]].tobytes() == raw, (kind, i)
+
+
+def test_a_payload_that_ends_with_a_block_header(gpu):
+    """Two fixed blocks and the three bits of a third, the last of the payload:
+    no symbol is left, and the member fails as the oracle's does."""
+    from oracle import oracle
+
+    for n in (6, 41, 3000):
+        bits = []
+
+        def code(value, width):  # Huffman codes go most significant bit first
+            bits.extend((value >> i) & 1 for i in range(width - 1, -1, -1))
+
+        for lits in (n, n % 5):
+            bits += [0, 1, 0]  # not the last, fixed codes
+            if lits == n:
+                code(0x190 + 7, 9)
+            for i in range(lits):
+                code(0x30 + i * 7 % 144, 8)
+            code(0, 7)
+        bits += [0, 1, 0]
+        assert len(bits) % 8 == 0
+        payload = np.packbits(np.array(bits, np.uint8), bitorder="little").tobytes()
+        data, spans = _file([(payload, bytes(n + n % 5 + 1))])
+        with pytest.raises(oracle.OracleError) as oe:
+            oracle.inflate_batch(data, spans)
+        with pytest.raises(gpu.FrtError) as ge:
+            gpu.CudaCodec(0).inflate_batch_device(data, spans)
+        assert (ge.value.code, ge.value.offset) == (oe.value.code, oe.value.offset)
