@@ -1523,7 +1523,8 @@ bool spread_launch(frt_inflate_tuning &t, u64 n, u32 *grid)
 {
     const int v = t.spread_variant >= 0 ? t.spread_variant : t.variant;
     if (kVariants[v].info.chains != 1 || n == 0) return false;
-    if ((t.warps_per_cta <= 1 || kVariants[v].team) && v == t.variant) return false;
+    if (kVariants[t.variant].team) return false; // a CTA per member already, and the shortest for a member alone
+    if (t.warps_per_cta <= 1 && v == t.variant) return false;
     int per_sm = g_spread_ctas[v].load(std::memory_order_relaxed);
     if (per_sm == 0) {
         frt_inflate_tuning one{v, 1, 0, 1, -1};
@@ -1564,7 +1565,7 @@ cudaError_t frt_launch_inflate_persistent(const u8 *in, const u64 *in_off, const
     // the tuned grid's warps gives a spread launch of n_cap one-warp CTAs
     frt_inflate_tuning t = tuned;
     // (a team variant needs no spreading: a CTA per member at most)
-    if (kVariants[t.variant].team && n_cap < grid) grid = (u32)(n_cap ? n_cap : 1);
+    if (kVariants[t.variant].team) grid = n_cap < grid ? (u32)(n_cap ? n_cap : 1) : grid;
     else if (n_cap < (u64)grid * (u64)tuned.warps_per_cta) spread_launch(t, n_cap, &grid);
     kVariants[t.variant].persistent<<<grid, cta_threads(t), frt_inflate_smem_bytes(t), s>>>(
         in, in_off, in_len, out, out_off, isize, crc_expect, status, produced, crc, order, n_ptr, n_cap,

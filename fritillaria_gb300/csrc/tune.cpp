@@ -429,6 +429,10 @@ int pick_spread_variant(frt_engine *e, int device, uint64_t members, frt_inflate
     const uint64_t few = members < (uint64_t)sms ? members : (uint64_t)sms;
     t.spread_variant = -1;
     if (few == 0) return FRT_OK;
+    if (frt::inflate_variant_team(t.variant)) { // the latency form itself: nothing to spread
+        t.spread_variant = t.variant;
+        return FRT_OK;
+    }
     double best = 0;
     int best_v = -1;
     for (int v = 0; v < frt_inflate_variant_count(); ++v) {

@@ -95,3 +95,22 @@ def test_a_payload_that_ends_with_a_block_header(gpu):
         with pytest.raises(gpu.FrtError) as ge:
             gpu.CudaCodec(0).inflate_batch_device(data, spans)
         assert (ge.value.code, ge.value.offset) == (oe.value.code, oe.value.offset)
+
+
+def test_a_tuning_with_a_spread_variant_keeps_the_team(gpu):
+    """Fewer members than the team's grid has warps, under a tuning that names a
+    serial spread variant: the bytes are zlib's, and the time of the launch is
+    the team's (a serial chain takes ten times as long)."""
+    torch = pytest.importorskip("torch")
+    from fritillaria_gb300 import synth
+
+    raw, bgzf = synth.short_read_bam(80_000, seed=5)
+    dev = torch.from_numpy(bgzf).to("cuda")
+    torch.cuda.synchronize()
+    eng = gpu.BatchEngine(0)
+    eng.bind_bam(dev.data_ptr(), dev.numel())
+    alone = eng.time_inflate(gpu.InflateTuning(0, 3, 0, 1, spread_variant=-1))[0]
+    assert eng.time_inflate(gpu.InflateTuning(0, 3, 0, 1, spread_variant=1))[0] < 3 * alone
+    eng.set_tuning(gpu.InflateTuning(0, 3, 0, 1, spread_variant=1))
+    eng.run()
+    assert eng.finish().status == 0 and np.array_equal(eng.inflated(), raw)
