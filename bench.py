@@ -670,7 +670,8 @@ def run_ours(args, rank, world, local):
             traffic = d.get("traffic_bytes_per_launch")
     roofline = {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 5), "traffic": traffic, "issue": issue_model(frt, eng, inflated, inflate_ms) if args.workload.startswith("short_reads") else None,
-                "kernel": "k_inflate_persistent (persistent warp-per-member inflate + CRC32/ISIZE verify)",
+                "kernel": "team::k_persistent (persistent CTA-per-member inflate + CRC32/ISIZE verify)" if tuning["variant"] == 0
+                else "k_inflate_persistent (persistent warp-per-member inflate + CRC32/ISIZE verify)",
                 "algorithmic_bytes_per_launch": inflate_bytes, "kernel_ms": round(inflate_ms, 3),
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
                 "pipeline": {"bytes": len(bgzf) + inflated + col_bytes, "ms": round(ms_step, 3),
@@ -998,7 +999,8 @@ def run_mixed(args, rank, world, local):
     achieved = inflate_bytes / (inflate_ms / 1e3) / 1e9
     roofline = {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 5), "traffic": None,
-                "kernel": "k_inflate_persistent (one persistent inflate over the members of all three files)",
+                "kernel": ("team::k_persistent" if tuning["variant"] == 0 else "k_inflate_persistent")
+                + " (one persistent inflate over the members of all three files)",
                 "algorithmic_bytes_per_launch": inflate_bytes, "kernel_ms": round(inflate_ms, 3),
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
                 "pipeline": {"bytes": blob.size + inflated + col_bytes, "ms": round(ms_step, 3),
@@ -1140,13 +1142,16 @@ def tick_breakdown(st: dict) -> dict:
 
 
 def issue_model(frt, eng, inflated: int, inflate_ms: float) -> dict | None:
-    """The inflate's second roofline: it is a serial Huffman chain per member,
-    so its bound is instruction issue, not HBM.  Warp instructions and DEFLATE
-    symbols per inflated byte come from the ncu capture and the symbol count in
-    profiles/inflate_issue.json; the issue peak is SMs x 4 schedulers x the SM
-    clock.  Also the chain model: warps in flight times each warp's symbol
-    rate, against one warp alone on an SM."""
-    ip = ROOT / "profiles" / "inflate_issue.json"
+    """The inflate's second roofline: its bound is instructions, not HBM.  Warp
+    instructions and DEFLATE symbols per inflated byte come from an ncu capture
+    and a symbol count: profiles/inflate_team_issue.json for the team form
+    (variant 0), profiles/inflate_issue.json for the serial variants; the issue
+    peak is SMs x 4 schedulers x the SM clock.  Also the chain model: warps in
+    flight times each warp's symbol rate, against a lone member's (team form:
+    its CTA's warps; serial form: one warp on an SM)."""
+    team = getattr(eng.tuning, "variant", None) == 0
+    name = "inflate_team_issue.json" if team else "inflate_issue.json"
+    ip = ROOT / "profiles" / name
     if not ip.exists() or inflate_ms <= 0:
         return None
     d = json.loads(ip.read_text())
@@ -1156,7 +1161,7 @@ def issue_model(frt, eng, inflated: int, inflate_ms: float) -> dict | None:
     peak = d["sms"] * d["schedulers_per_sm"] * d["sm_clock_hz"]
     instr = per_byte * inflated / secs
     t = eng.tuning
-    warps = int(d["sms"]) * int(t.warps_per_cta) * max(1, frt.inflate_ctas_per_sm(t))
+    warps = int(d["sms"]) * int(d.get("warps_per_cta", t.warps_per_cta)) * max(1, frt.inflate_ctas_per_sm(t))
     sym = sym_per_byte * inflated / secs
     return {"achieved": round(instr / 1e12, 4), "peak": round(peak / 1e12, 4), "unit": "T warp instructions/s",
             "frac": round(instr / peak, 4), "instructions_per_symbol": round(per_byte / sym_per_byte, 1),
@@ -1164,7 +1169,7 @@ def issue_model(frt, eng, inflated: int, inflate_ms: float) -> dict | None:
                       "per_warp_symbols_per_s": round(sym / warps / 1e6, 3),
                       "lone_warp_symbols_per_s": round(d["lone_warp_symbols_per_s"] / 1e6, 3),
                       "unit": "G symbols/s (total), M symbols/s (per warp)"},
-            "source": "profiles/inflate_issue.json (instructions and symbols per inflated byte of the 2M capture)"}
+            "source": f"profiles/{name} (instructions and symbols per inflated byte of the 2M capture)"}
 
 
 def run_serving(args, rank, world, local):
