@@ -203,7 +203,12 @@ __device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u6
     const u64 lo = min(me, ms + w * part), hi = min(me, lo + part);
     u16 *const place = scratch + (size_t)m * FRT_SCAN_CAP;
     u64 e = INF64;
-    if (lo < hi && hi > start) e = lo <= start ? start : find_start(buf, len, lo, hi, n_ref);
+    if (lo < hi && hi > start) {
+        // the part's lines on their way to L2 while its start is looked for: a
+        // hop of the walk then waits for L2, not for HBM
+        for (u64 at = lo + 128ull * lane; at < hi; at += 128ull * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(buf + at));
+        e = lo <= start ? start : find_start(buf, len, lo, hi, n_ref);
+    }
     if (lane == 0) {
         Seg s{e, 0u, 1, 1};
         if (e != INF64) s = whole ? walk_record(buf, len, e, hi, ms, place, FRT_SCAN_CAP) : walk_record(buf, len, e, hi, ms, s_rec[w], SPEC_CAP);
