@@ -146,12 +146,15 @@ __device__ u64 find_start(const u8 *buf, u64 len, u64 lo, u64 hi, int n_ref)
         }
 #pragma unroll
         for (u32 g = 0; g < 4u; ++g) {
-            u32 first = 4;
+            u32 may = 0; // offsets whose ref_id passes; tested apart, as few do
 #pragma unroll
-            for (u32 k = 0; k < 4u; ++k) {
-                const u32 ref = k ? __funnelshift_r(w0[g], w1[g], 8u * k) : w0[g];
+            for (u32 k = 0; k < 4u; ++k) may |= ((k ? __funnelshift_r(w0[g], w1[g], 8u * k) : w0[g]) + 1u <= (u32)n_ref ? 1u : 0u) << k;
+            if (!__any_sync(FRT_FULL_MASK, may)) continue;
+            u32 first = 4;
+            for (; may && first == 4; may &= may - 1) {
+                const u32 k = (u32)__ffs(may) - 1u;
                 const long long ps = base + 128 * g + 4ll * lane + k;
-                if (first == 4 && ps >= (long long)lo && ps < (long long)hi && ref + 1u <= (u32)n_ref) {
+                if (ps >= (long long)lo && ps < (long long)hi) {
                     const u64 p = (u64)ps;
                     bool ok = plausible(buf, len, p, n_ref);
                     if (ok) {
