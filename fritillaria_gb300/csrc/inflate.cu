@@ -31,6 +31,7 @@
 // reference kernel (crates/fritillaria-cuda/kernels/inflate.cu:78-458), so a
 // stream it rejects is rejected here with the same code.
 
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <mutex>
@@ -1373,7 +1374,8 @@ template <int NW, int PER_SM> Variant make_team_variant()
 // queue trade shared memory against bursts per member; a register cap (80:
 // no spills; 72, 64 and 56: up to ~120 spilled bytes) lets more CTAs fit an SM.
 // Variant 0 is the default before any tuning: the team form, one member per
-// CTA whatever CTA width a tuning names.
+// CTA whatever CTA width a tuning names (a launch of many short members takes
+// kShort below in its place).
 const Variant kVariants[] = {
     make_team_variant<12, 2>(),
     make_variant<Cfg<10, 8, 2048, 384>>(),     make_variant<Cfg<9, 8, 2048, 384>>(),
@@ -1541,12 +1543,54 @@ bool spread_launch(frt_inflate_tuning &t, u64 n, u32 *grid)
 }
 } // namespace
 
+namespace {
+// CTAs of a team variant, and of the serial form's kShort tuning, an SM holds
+// (0: not yet asked).
+std::atomic<int> g_team_ctas[kNumVariants], g_short_ctas;
+
+int ctas_of(std::atomic<int> &known, const frt_inflate_tuning &t)
+{
+    int per_sm = known.load(std::memory_order_relaxed);
+    if (per_sm == 0) {
+        per_sm = frt_inflate_ctas_per_sm(t);
+        known.store(per_sm > 0 ? per_sm : -1, std::memory_order_relaxed);
+    }
+    return per_sm;
+}
+
+// Short members go to the serial form where each CTA of the team form would
+// have several.  Whatever a member holds, a team takes some 28 us for it (its
+// tables and the barriers of each phase), one after another; a warp of the
+// serial form takes 75 us for a record of short reads, 12 times as many warps
+// run side by side, and its time grows with the member.  Measured on members of
+// 330 / 1,000 / 2,000 / 2,600 / 4,000 bytes of short reads, team and serial, us:
+//      700 of them    90   75 |   92  125 |   94  188 |   94  236 |   98  344
+//    1,000           117   75 |  122  123 |  123  188 |  125  238 |  131  345
+//    2,000           202   86 |  213  139 |  223  213 |  227  270 |  241  397
+//    4,000           390  157 |  410  262 |  415  409 |  422  520 |  449  767
+//   40,000          3694 1174 | 3901 1964 | 4042 3077 | 4096 3947 | 4355 5810
+// so the line lies at 190 compressed bytes for each member a CTA has, up to 7.
+constexpr frt_inflate_tuning kShort{1, 3, 0, 1, -1};
+constexpr u64 kShortBytes = 190, kShortShare = 7;
+
+// `grid` CTAs of a team variant, n members of in_bytes in all.
+bool short_members(u64 grid, u64 n, u64 in_bytes)
+{
+    const u64 share = grid ? n / grid : 0;
+    return share >= 2 && in_bytes <= n * kShortBytes * std::min(share, kShortShare);
+}
+} // namespace
+
 cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                        const u64 *out_off, const u32 *out_cap, u32 *status, u32 *produced,
-                                       u32 *crc, u32 n, const frt_inflate_tuning &tuned, cudaStream_t s)
+                                       u32 *crc, u32 n, u64 in_bytes, const frt_inflate_tuning &tuned, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
     frt_inflate_tuning t = tuned;
+    if (kVariants[t.variant].team) {
+        const int per_sm = ctas_of(g_team_ctas[t.variant], {t.variant, 1, 0, 1, -1});
+        if (per_sm > 0 && short_members((u64)per_sm * (u64)sm_count(), n, in_bytes)) t = kShort;
+    }
     u32 unused = 0;
     spread_launch(t, n, &unused);
     const u32 w = kVariants[t.variant].team ? 1u : (u32)t.warps_per_cta * (u32)kVariants[t.variant].info.chains; // members per CTA
@@ -1558,15 +1602,22 @@ cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u3
 cudaError_t frt_launch_inflate_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                           const u64 *out_off, const u32 *isize, const u32 *crc_expect, u32 *status,
                                           u32 *produced, u32 *crc, const u32 *order, const u64 *n_ptr, u64 n_cap,
-                                          u64 out_capacity, u32 *queue_head, u32 grid, unsigned long long *block_err,
-                                          const frt_inflate_tuning &tuned, cudaStream_t s)
+                                          u64 in_bytes, u64 out_capacity, u32 *queue_head, u32 grid,
+                                          unsigned long long *block_err, const frt_inflate_tuning &tuned, cudaStream_t s)
 {
     // n_cap bounds the members (the device count may be lower): fewer than
     // the tuned grid's warps gives a spread launch of n_cap one-warp CTAs
     frt_inflate_tuning t = tuned;
+    if (kVariants[t.variant].team && short_members(grid, n_cap, in_bytes)) {
+        const int per_sm = ctas_of(g_short_ctas, kShort);
+        if (per_sm > 0) {
+            t = kShort;
+            grid = (u32)per_sm * (u32)sm_count();
+        }
+    }
     // (a team variant needs no spreading: a CTA per member at most)
     if (kVariants[t.variant].team) grid = n_cap < grid ? (u32)(n_cap ? n_cap : 1) : grid;
-    else if (n_cap < (u64)grid * (u64)tuned.warps_per_cta) spread_launch(t, n_cap, &grid);
+    else if (n_cap < (u64)grid * (u64)t.warps_per_cta) spread_launch(t, n_cap, &grid);
     kVariants[t.variant].persistent<<<grid, cta_threads(t), frt_inflate_smem_bytes(t), s>>>(
         in, in_off, in_len, out, out_off, isize, crc_expect, status, produced, crc, order, n_ptr, n_cap,
         out_capacity, queue_head, (u32)t.queue_chunk, block_err);

@@ -328,7 +328,7 @@ int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const fr
     std::vector<uint32_t> plan32(2 * n);
     uint64_t *in_off = plan64.data(), *out_off = plan64.data() + n;
     uint32_t *in_len = plan32.data(), *cap = plan32.data() + n;
-    uint64_t total = 0;
+    uint64_t total = 0, in_bytes = 0;
     for (size_t i = 0; i < n; ++i) {
         const frt_span &s = spans[i];
         if (s.isize > 65536u) {
@@ -346,6 +346,7 @@ int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const fr
         out_off[i] = total;
         cap[i] = s.isize;
         total += s.isize;
+        in_bytes += s.payload_len;
     }
     out_off[n] = total;
     DeviceGuard g(c->device);
@@ -392,7 +393,7 @@ int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const fr
     if ((e = cudaMemcpyAsync(work, plan64.data(), 8 * (2 * n + 1), cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e, "uploading plan");
     if ((e = cudaMemcpyAsync(d_in_len, plan32.data(), 8 * n, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e, "uploading plan");
     if ((e = frt_launch_inflate_members(input, d_in_off, d_in_len, output, d_out_off, d_cap, d_status, d_produced,
-                                        d_crc, (u32)n, c->tuning, st)) != cudaSuccess)
+                                        d_crc, (u32)n, in_bytes, c->tuning, st)) != cudaSuccess)
         return fail(e, "launching inflate");
     std::vector<uint32_t> res(3 * n);
     if (n && (e = cudaMemcpyAsync(res.data(), d_status, 12 * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return fail(e, "downloading status");
