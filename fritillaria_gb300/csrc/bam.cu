@@ -7,12 +7,12 @@
 // (crates/fritillaria-cuda/kernels/bam_decode.cu:154-216).  This file removes
 // that serial walk:
 //
-//   1. spec: a CTA per member searches the member for its first plausible
-//      record start (a 512-offset sieve with a strict validator: block_size,
+//   1. spec: a CTA per member (a warp, where the members are many) searches
+//      the member for its first plausible record start (a 512-offset sieve with a strict validator: block_size,
 //      refID/next_refID range, positions, NUL-terminated name, declared fields
 //      fit, and the next two records validate too) and walks the chain from
-//      there to the member end, recording record offsets in scratch -- an
-//      eighth of the member a warp, the parts joined where walks meet;
+//      there to the member end, recording record offsets in scratch -- a CTA
+//      an eighth of the member a warp, the parts joined where walks meet;
 //   2. reconcile: one CTA proves the chain.  The true arrival into member m is
 //      max(start, lands of earlier members that hold a record start) -- a
 //      prefix max, computed block-wide.  Member m is proven when its
@@ -191,7 +191,8 @@ constexpr u32 SPEC_CAP = (SPEC_PART + 35) / 36;        // most record starts in 
 // searches its part and walks it from what it found.  One thread then follows
 // the walks from the member's first start: where a walk lands on the start its
 // part's warp found, that part's records are the chain's; elsewhere the part
-// is walked again from the landing.  The result is the one walk's.
+// is walked again from the landing.  The result is the one walk's
+// (spec_member_warp).
 __device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u64 start, int n_ref, u64 *entry,
                             u32 *count, u64 *land, u8 *flags, u16 *scratch)
 {
@@ -256,32 +257,69 @@ __device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u6
     for (u32 i = lane; i < s_count[w]; i += 32) place[before + i] = s_rec[w][i];
 }
 
-// Phase 1.  One CTA per member.
+// The same by one warp: eight searches and walks take more of a full GPU's time
+// than one does.
+__device__ void spec_member_warp(const u8 *buf, u64 len, const u64 *starts, u32 m, u64 start, int n_ref, u64 *entry,
+                                 u32 *count, u64 *land, u8 *flags, u16 *scratch)
+{
+    const u64 ms = starts[m], me = starts[m + 1];
+    u64 e = INF64;
+    if (ms < me && me > start) e = ms <= start ? start : find_start(buf, len, ms, me, n_ref);
+    if (lane_id() == 0) {
+        Seg s{e, 0u, 1, 1};
+        if (e != INF64) s = walk_record(buf, len, e, me, ms, scratch + (size_t)m * FRT_SCAN_CAP, FRT_SCAN_CAP);
+        entry[m] = e;
+        count[m] = s.count;
+        land[m] = e == INF64 ? 0ull : s.land;
+        flags[m] = (u8)((s.complete ? 1 : 0) | (s.valid ? 2 : 0));
+    }
+}
+
+// Whether n members of `bytes` in all are scanned a CTA a member.  Its gain is
+// one member's latency, which a warp each hides once there are many; its cost
+// is in the searches, which short members have little else to do but.
+// Measured (whole record stage, us, a CTA and a warp a member):
+//   65,280 bytes:  1,000 members 158 and 224,  4,000 364 and 382,  10,000 798 and 765
+//   16,000 bytes:    152 members  78 and  90,  1,000  81 and  94,   2,000 109 and 105,  40,000 1,215 and 775
+//    4,000 bytes:    620 members  64 and  66,  1,000  70 and  64,  40,000   826 and 351
+//      330 bytes:    700 members  55 and  51, 40,000 541 and 221
+// so the line lies where ten members' number passes a member's mean bytes.
+constexpr u64 SPEC_MANY = 10;
+bool spec_by_cta(u64 n, u64 bytes) { return SPEC_MANY * n <= bytes / n; }
+
+// Phase 1.  One CTA per member, or one warp.
+template <bool BY_CTA>
 __global__ void __launch_bounds__(32 * SPEC_WARPS)
 k_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n_members, u64 start, int n_ref, u64 *entry, u32 *count,
            u64 *land, u8 *flags, u16 *scratch, const u64 *start_dev, const int *nref_dev)
 {
-    u32 m = blockIdx.x;
+    const u32 m = BY_CTA ? blockIdx.x : blockIdx.x * SPEC_WARPS + threadIdx.x / 32;
     if (m >= n_members) return;
     if (start_dev) start = *start_dev;
     if (nref_dev) n_ref = *nref_dev < 0 ? (1 << 24) : *nref_dev;
-    spec_member(buf, len, starts, m, start, n_ref, entry, count, land, flags, scratch);
+    if (BY_CTA) spec_member(buf, len, starts, m, start, n_ref, entry, count, land, flags, scratch);
+    else spec_member_warp(buf, len, starts, m, start, n_ref, entry, count, land, flags, scratch);
 }
 
 // Phase 1 over many segments (independent record chains, each over its own
 // members): segment s owns members [seg[s].m0, seg[s].m0 + seg[s].n) of the
 // per-member arrays and the n + 1 starts at starts + seg[s].m0 + s.
+template <bool BY_CTA>
 __global__ void __launch_bounds__(32 * SPEC_WARPS)
 k_bam_spec_seg(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_total, int n_ref, const u64 *starts,
                u64 *entry, u32 *count, u64 *land, u8 *flags, u16 *scratch)
 {
-    u32 g = blockIdx.x;
+    const u32 g = BY_CTA ? blockIdx.x : blockIdx.x * SPEC_WARPS + threadIdx.x / 32;
     if (g >= n_total) return;
     u32 si = seg_of[g];
     FrtScanSeg sg = seg[si];
     u32 j = g - sg.m0;
-    spec_member(buf, sg.len, starts + sg.m0 + si, j, sg.start, n_ref, entry + sg.m0, count + sg.m0, land + sg.m0,
-                flags + sg.m0, scratch + (size_t)sg.m0 * FRT_SCAN_CAP);
+    if (BY_CTA)
+        spec_member(buf, sg.len, starts + sg.m0 + si, j, sg.start, n_ref, entry + sg.m0, count + sg.m0, land + sg.m0,
+                    flags + sg.m0, scratch + (size_t)sg.m0 * FRT_SCAN_CAP);
+    else
+        spec_member_warp(buf, sg.len, starts + sg.m0 + si, j, sg.start, n_ref, entry + sg.m0, count + sg.m0, land + sg.m0,
+                         flags + sg.m0, scratch + (size_t)sg.m0 * FRT_SCAN_CAP);
 }
 
 // Phase 2 for one record chain, by one CTA of 1024 threads.  totals =
@@ -862,8 +900,12 @@ cudaError_t frt_launch_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n
                                 const int *nref_dev)
 {
     if (n == 0) return cudaSuccess;
-    k_bam_spec<<<n, 32 * SPEC_WARPS, 0, s>>>(buf, len, starts, n, start, n_ref, entry, count, land, flags, scratch,
-                                           start_dev, nref_dev);
+    if (spec_by_cta(n, len))
+        k_bam_spec<true><<<n, 32 * SPEC_WARPS, 0, s>>>(buf, len, starts, n, start, n_ref, entry, count, land, flags,
+                                                       scratch, start_dev, nref_dev);
+    else
+        k_bam_spec<false><<<(n + SPEC_WARPS - 1) / SPEC_WARPS, 32 * SPEC_WARPS, 0, s>>>(
+            buf, len, starts, n, start, n_ref, entry, count, land, flags, scratch, start_dev, nref_dev);
     return cudaGetLastError();
 }
 
@@ -887,13 +929,18 @@ cudaError_t frt_launch_bam_decode(const u8 *buf, const u64 *starts, const u64 *c
 
 size_t frt_scan_partials_len(u64 n) { return (size_t)(n / 4096 + 1); }
 
-cudaError_t frt_launch_region_scan(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_segs, u32 n_total,
-                                   int n_ref, const u64 *starts, const u64 *coff, u64 *entry, u32 *count, u64 *land,
+cudaError_t frt_launch_region_scan(const u8 *buf, u64 len, const FrtScanSeg *seg, const u32 *seg_of, u32 n_segs,
+                                   u32 n_total, int n_ref, const u64 *starts, const u64 *coff, u64 *entry, u32 *count, u64 *land,
                                    u8 *flags, u16 *scratch, u32 *first_index, u64 *totals, u32 *kept, cudaStream_t s)
 {
     if (n_total == 0 || n_segs == 0) return cudaSuccess;
     unsigned g = (n_total + 7) / 8; // warp-per-member grids below
-    k_bam_spec_seg<<<n_total, 32 * SPEC_WARPS, 0, s>>>(buf, seg, seg_of, n_total, n_ref, starts, entry, count, land, flags, scratch);
+    if (spec_by_cta(n_total, len))
+        k_bam_spec_seg<true><<<n_total, 32 * SPEC_WARPS, 0, s>>>(buf, seg, seg_of, n_total, n_ref, starts, entry, count,
+                                                                 land, flags, scratch);
+    else
+        k_bam_spec_seg<false><<<g, 32 * SPEC_WARPS, 0, s>>>(buf, seg, seg_of, n_total, n_ref, starts, entry, count, land,
+                                                            flags, scratch);
     k_bam_reconcile_seg<<<n_segs, 1024, 0, s>>>(buf, seg, starts, entry, count, land, flags, scratch, first_index,
                                                 totals);
     k_region_count<<<g, 256, 0, s>>>(buf, seg, seg_of, n_total, starts, coff, count, scratch, kept);

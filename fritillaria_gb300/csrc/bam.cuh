@@ -69,8 +69,9 @@ struct FrtRegionColumns {
     u32 *request;
 };
 
-cudaError_t frt_launch_region_scan(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_segs, u32 n_total,
-                                   int n_ref, const u64 *starts, const u64 *coff, u64 *entry, u32 *count, u64 *land,
+// len: the buffer's bytes.
+cudaError_t frt_launch_region_scan(const u8 *buf, u64 len, const FrtScanSeg *seg, const u32 *seg_of, u32 n_segs,
+                                   u32 n_total, int n_ref, const u64 *starts, const u64 *coff, u64 *entry, u32 *count, u64 *land,
                                    u8 *flags, u16 *scratch, u32 *first_index, u64 *totals, u32 *kept, cudaStream_t s);
 cudaError_t frt_launch_region_emit(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_total,
                                    const u64 *starts, const u64 *coff, const u32 *count, const u16 *scratch,

@@ -343,7 +343,7 @@ int launch_tick(frt_server *sv, std::vector<SrvReq *> &batch, frt_error *err)
     cudaEventRecord(t->ev_inflated, st);
     int32_t n_ref = 0; // bounds refID in the record-start test
     for (SrvReq *r : batch) n_ref = std::max(n_ref, sv->files[r->file].n_ref < 0 ? (1 << 24) : sv->files[r->file].n_ref);
-    if ((e = frt_launch_region_scan(t->arena, segs, seg_of, ns, n, n_ref, starts, coff, entry, count, land, flags,
+    if ((e = frt_launch_region_scan(t->arena, pl.arena_bytes, segs, seg_of, ns, n, n_ref, starts, coff, entry, count, land, flags,
                                     scratch, first, totals, kept, st)) != cudaSuccess)
         return cuda_fail(err, e, "launching the region scan");
     if ((e = frt_launch_scan_u32(kept, n, parts, kept_first, tot32, st)) != cudaSuccess)
