@@ -135,6 +135,7 @@ __device__ Seg walk_record(const u8 *buf, u64 len, u64 from, u64 until, u64 msta
 __device__ u64 find_start(const u8 *buf, u64 len, u64 lo, u64 hi, int n_ref)
 {
     const u32 lane = lane_id();
+    hi = min(hi, len); // no record starts past the batch
     const long long A = (long long)(((uintptr_t)(buf + lo) & ~(uintptr_t)3) - (uintptr_t)buf);
     for (long long base = A; base < (long long)hi; base += 512) {
         u32 w0[4], w1[4];
@@ -209,8 +210,9 @@ __device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u6
     u64 e = INF64;
     if (lo < hi && hi > start) {
         // the part's lines on their way to L2 while its start is looked for: a
-        // hop of the walk then waits for L2, not for HBM
-        for (u64 at = lo + 128ull * lane; at < hi; at += 128ull * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(buf + at));
+        // hop of the walk then waits for L2, not for HBM (offsets are the caller's:
+        // none past the batch)
+        for (u64 at = lo + 128ull * lane; at < min(hi, len); at += 128ull * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(buf + at));
         e = lo <= start ? start : find_start(buf, len, lo, hi, n_ref);
     }
     if (lane == 0) {

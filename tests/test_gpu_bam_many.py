@@ -26,3 +26,17 @@ def test_many_short_members_cost_little_more(gpu):
         pos[payload] = eng.column("pos")
     assert np.array_equal(pos[1000], pos[65_280])
     assert took[1000] < 3 * took[65_280]
+
+
+def test_offsets_past_the_batch_reach_no_byte_past_it(gpu):
+    """Members that end up to 64 KiB past the batch are refused; the scan that
+    runs before the refusal stays inside the batch, its prefetches too."""
+    torch = pytest.importorskip("torch")
+    raw, _ = synth.raw_bam("short_reads", 400, seed=5)
+    dev = torch.from_numpy(raw).to("cuda")
+    out = torch.zeros(1000, dtype=torch.int64, device="cuda")
+    for offsets in ([0, 65_000, 65_000 + 60_000], [65_000, 130_000], [70_000, 10]):
+        offs = torch.tensor(offsets, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        with pytest.raises(gpu.InvalidArgument):
+            gpu.bam_scan_noalloc(dev.data_ptr(), 70_000, offs.data_ptr(), len(offsets) - 1, 0, out.data_ptr(), 1000, n_ref=1)
