@@ -1366,7 +1366,7 @@ template <int NW, int PER_SM> Variant make_team_variant()
     using S = team::Smem<NW>;
     return {{(int32_t)team::LR, (int32_t)team::DR, (int32_t)((team::OUT_MAX / NW + 31) / 32 * 32), (int32_t)team::GROUP_MATCHES,
              65536 / (32 * NW * PER_SM) / 8 * 8, 1, 0, (uint64_t)((sizeof(S) + NW - 1) / NW)},
-            team::k_members<NW, PER_SM>, team::k_persistent<NW, PER_SM>, (u32)NW};
+            nullptr, team::k_persistent<NW, PER_SM>, (u32)NW}; // one kernel for both forms
 }
 
 // The compiled variants: the table roots trade shared memory (members in
@@ -1455,7 +1455,7 @@ cudaError_t frt_inflate_prepare()
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
     for (const Variant &v : kVariants) {
-        if ((e = cudaFuncSetAttribute(v.members, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess)
+        if (v.members && (e = cudaFuncSetAttribute(v.members, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess)
             return e;
         if ((e = cudaFuncSetAttribute(v.persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess)
             return e;
@@ -1583,7 +1583,8 @@ bool short_members(u64 grid, u64 n, u64 in_bytes)
 
 cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                        const u64 *out_off, const u32 *out_cap, u32 *status, u32 *produced,
-                                       u32 *crc, u32 n, u64 in_bytes, const frt_inflate_tuning &tuned, cudaStream_t s)
+                                       u32 *crc, u32 n, u64 in_bytes, u32 *queue_head, const frt_inflate_tuning &tuned,
+                                       cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
     frt_inflate_tuning t = tuned;
@@ -1593,7 +1594,15 @@ cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u3
     }
     u32 unused = 0;
     spread_launch(t, n, &unused);
-    const u32 w = kVariants[t.variant].team ? 1u : (u32)t.warps_per_cta * (u32)kVariants[t.variant].info.chains; // members per CTA
+    if (kVariants[t.variant].team) {
+        const int per_sm = ctas_of(g_team_ctas[t.variant], {t.variant, 1, 0, 1, -1});
+        const u64 slots = per_sm > 0 ? (u64)per_sm * (u64)sm_count() : 1;
+        kVariants[t.variant].persistent<<<(u32)std::min<u64>(n, slots), cta_threads(t), frt_inflate_smem_bytes(t), s>>>(
+            in, in_off, in_len, out, out_off, out_cap, nullptr, status, produced, crc, nullptr, nullptr, n, ~0ull,
+            queue_head, 1u, nullptr);
+        return cudaGetLastError();
+    }
+    const u32 w = (u32)t.warps_per_cta * (u32)kVariants[t.variant].info.chains; // members per CTA
     kVariants[t.variant].members<<<(n + w - 1) / w, cta_threads(t), frt_inflate_smem_bytes(t), s>>>(
         in, in_off, in_len, out, out_off, out_cap, status, produced, crc, n);
     return cudaGetLastError();

@@ -23,10 +23,11 @@ int frt_inflate_persistent_grid(const frt_inflate_tuning &t);
 
 cudaError_t frt_inflate_prepare();
 // in_bytes: the compressed bytes of the launch's members, or about that many
-// (their mean length says which form takes them).
+// (their mean length says which form takes them).  queue_head: a word that is 0.
 cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                        const u64 *out_off, const u32 *out_cap, u32 *status, u32 *produced,
-                                       u32 *crc, u32 n, u64 in_bytes, const frt_inflate_tuning &t, cudaStream_t s);
+                                       u32 *crc, u32 n, u64 in_bytes, u32 *queue_head, const frt_inflate_tuning &t,
+                                       cudaStream_t s);
 cudaError_t frt_launch_inflate_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                           const u64 *out_off, const u32 *isize, const u32 *crc_expect, u32 *status,
                                           u32 *produced, u32 *crc, const u32 *order, const u64 *n_ptr, u64 n_cap,

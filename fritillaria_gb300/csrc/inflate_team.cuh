@@ -111,6 +111,8 @@ template <int NW> struct Smem {
     Code lit, dist;
     u32 sh[8]; // uniform values handed from one thread to the team
     u32 fail, hint;
+    u32 brief, blocks; // bits a block below which the member is the serial form's; its blocks so far
+    u32 list[NW], listed; // members that wait for the serial form
     u16 lsorted[288], dsorted[32];
     u8 lens[320];
 };
@@ -771,6 +773,21 @@ __device__ __forceinline__ u32 stage_from(Smem<NW> *sm, const u32 *base, u32 wor
     return skew - 32u * w0;
 }
 
+// A block costs the team some 26 us (its tables, the staging, the barriers) and
+// 0.5 us a kilobit, a warp of the serial form 21 and 15; a CTA has twelve of
+// those, which slow each other down twofold.  So members of several short
+// blocks are the serial form's, where enough of them are at hand: by BRIEF bits
+// a block for each further member a CTA has, up to BRIEF_SHARE.  Measured on
+// short-read members of 65,280 bytes by zlib's memLevel (bits a block), in ms
+// the team alone, the serial variant, and the two as they are chosen:
+//                  1,000 members       4,000               10,000
+//   1  (1,200)   22.9  10.2   9.3    83.5  23.8  22.6    203   49.3  40.8
+//   2  (2,400)   11.3   7.1   6.8    41.1  16.3  16.1    100   33.4  28.7
+//   3  (4,800)    5.8   5.7   5.8    21.0  12.5  13.0     51.0 26.2  23.3
+//   4  (9,600)    3.1   5.0   3.1    11.4  11.1  11.9     27.6 23.3  21.2
+//   5 (19,000)    1.7   4.8   1.7     6.2  10.9   6.3     15.0 22.1  15.1
+constexpr u32 BRIEF = 1500, BRIEF_SHARE = 7;
+
 // One Huffman block from bit `bitpos` (its tables built): bitpos moves past
 // its end-of-block code, pos over its bytes.  `off` is the staged place of bit
 // 0 (stage_from).  False (uniform): the serial form is to take the member.
@@ -880,7 +897,11 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
         pos += tot;
         __syncthreads();
         if (how == F_END) {
-            if (!last_block && tid == 0) sm->hint = bitpos - block_at + (bitpos - block_at) / 16u;
+            if (!last_block && tid == 0) {
+                sm->hint = bitpos - block_at + (bitpos - block_at) / 16u;
+                const u32 blocks = ++sm->blocks;
+                if (blocks >= 2 && bitpos < blocks * sm->brief && total - bitpos > 2 * sm->brief) sm->fail = 1;
+            }
             return true;
         }
         off = stage_from<NW>(sm, base, words, skew, bitpos);
@@ -901,9 +922,11 @@ __device__ bool member(Smem<NW> *sm, const u8 *in, u32 in_len, u8 *to, u32 cap, 
     const u32 skew = 8u * (u32)((u64)in & 3ull), total = 8u * in_len;
     const u32 words = (skew + total + 31u) / 32u; // only words that hold payload are read
     u32 bitpos = 0, pos = 0;
+    if (tid == 0) sm->blocks = 0;
     while (true) {
         if (bitpos + 3 > total) return false;
         const u32 off = stage_from<NW>(sm, base, words, skew, bitpos);
+        if (sm->fail) return false;
         const u32 v = bits_at(sm->stage, off + bitpos);
         const bool fin = v & 1u;
         const u32 type = (v >> 1) & 3u;
@@ -953,24 +976,6 @@ template <int NW> __device__ __forceinline__ void clear_marks(Smem<NW> *sm)
     }
 }
 
-using Serial = Cfg<9, 7, 1024, 192>;
-
-// The serial form on warp 0, in the output buffer's place.
-template <int NW>
-__device__ __noinline__ u32 member_serial(Smem<NW> *sm, const u8 *in, u32 in_len, u8 *to, u32 cap, u32 *produced,
-                                          u32 *crc_out)
-{
-    static_assert(sizeof(WarpSmem<Serial>) <= sizeof(sm->out), "the serial form's state fits the output buffer");
-    __syncthreads();
-    u32 st = INF_OK, p = 0, c = 0;
-    if (threadIdx.x < 32) st = inflate_member_warp<Serial>(in, in_len, to, cap, (WarpSmem<Serial> *)sm->out, &p, &c);
-    clear_marks<NW>(sm);
-    __syncthreads();
-    *produced = p;
-    *crc_out = c;
-    return st; // valid in warp 0
-}
-
 template <int NW> __device__ __forceinline__ void setup(Smem<NW> *sm)
 {
     const u32 tid = threadIdx.x, NT = Smem<NW>::NT;
@@ -984,31 +989,63 @@ template <int NW> __device__ __forceinline__ void setup(Smem<NW> *sm)
     __syncthreads();
 }
 
-// Plain form: one CTA per member, members in span order.
-template <int NW, int PER_SM>
-__global__ void __launch_bounds__(32 * NW, PER_SM)
-k_members(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out, const u64 *out_off, const u32 *out_cap,
-          u32 *status, u32 *produced, u32 *crc, u32 n)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    Smem<NW> *sm = (Smem<NW> *)smem;
-    const u32 m = blockIdx.x;
-    if (m >= n) return;
-    setup<NW>(sm);
-    u32 p = 0, c = 0, st = INF_OK;
-    const u8 *src = in + in_off[m];
-    u8 *to = out + out_off[m];
-    if (!member<NW>(sm, src, in_len[m], to, out_cap[m], &p, &c))
-        st = member_serial<NW>(sm, src, in_len[m], to, out_cap[m], &p, &c);
-    if (threadIdx.x == 0) {
+// A launch's members.
+struct Job {
+    const u8 *in;
+    const u64 *in_off;
+    const u32 *in_len;
+    u8 *out;
+    const u64 *out_off;
+    const u32 *cap;
+    const u32 *crc_expect; // null: the caller checks
+    u32 *status, *produced, *crc;
+    unsigned long long *block_err;
+    // A member's result, by one thread: with crc_expect, checked against its
+    // trailer as in k_inflate_persistent.
+    __device__ __forceinline__ void put(u32 m, u32 st, u32 p, u32 c) const
+    {
         status[m] = st;
         produced[m] = p;
         crc[m] = st == INF_OK ? c : 0u;
+        if (!crc_expect) return;
+        const unsigned long long code = st != INF_OK ? 5ull : (p != cap[m] ? 4ull : (c != crc_expect[m] ? 3ull : 0ull));
+        if (code) atomicMin(block_err, ((unsigned long long)m << 8) | code);
     }
+};
+
+using Serial = Cfg<9, 7, 1024, 192>;
+
+// The `listed` members of sm->list by the serial form, a warp each, in the place
+// of the output and the block's tables.
+template <int NW> __device__ __noinline__ void run_listed(Smem<NW> *sm, const Job &job, u32 listed)
+{
+    static_assert(NW * sizeof(WarpSmem<Serial>) <= offsetof(Smem<NW>, tab) + 4 * EXTRA_AT, "the serial form's states leave the rest");
+    __syncthreads(); // the list is whole, and nothing else in use
+    const u32 warp = threadIdx.x / 32;
+    if (warp < listed) {
+        const u32 m = sm->list[warp];
+        u32 p = 0, c = 0;
+        const u32 st = inflate_member_warp<Serial>(job.in + job.in_off[m], job.in_len[m], job.out + job.out_off[m], job.cap[m],
+                                                   (WarpSmem<Serial> *)sm->out + warp, &p, &c);
+        if (lane_id() == 0) job.put(m, st, p, c);
+    }
+    __syncthreads();
+    clear_marks<NW>(sm);
+    if (threadIdx.x == 0) sm->listed = 0;
+    __syncthreads();
 }
 
-// Batched form: the persistent grid and the trailer check of
-// k_inflate_persistent, a CTA per popped member.
+// A grid of CTAs that pull members from a queue (`order`, or in their order)
+// through an atomic head, `chunk` a pop; a grid of a CTA for each member, where
+// no order is given, takes one each and no queue (one that is, as the slices of
+// a file still on its way here, shares the SMs with others: a CTA that runs
+// takes members of those that do not yet).
+//
+// A member the team does not take is the serial form's.  Where a CTA has
+// several members to do, such members wait on a list until there is one for
+// each warp (alone, one leaves eleven warps idle).  One that is alone on the
+// list at the end is the team's as far as it goes.  Where there are members to
+// fill every CTA's list, the next ones after two in a row are listed untried.
 template <int NW, int PER_SM>
 __global__ void __launch_bounds__(32 * NW, PER_SM)
 k_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out, const u64 *out_off, const u32 *isize,
@@ -1017,37 +1054,64 @@ k_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out, const 
 {
     extern __shared__ __align__(16) unsigned char smem[];
     Smem<NW> *sm = (Smem<NW> *)smem;
-    const u64 n64 = *n_ptr;
+    const u64 n64 = n_ptr ? *n_ptr : n_cap;
     const u32 n = (u32)(n64 < n_cap ? n64 : n_cap);
     if (chunk == 0) chunk = 1;
+    const Job job{in, in_off, in_len, out, out_off, isize, crc_expect, status, produced, crc, block_err};
+    const bool queue = order || gridDim.x < n;
     setup<NW>(sm);
+    if (threadIdx.x == 0) {
+        sm->brief = queue ? BRIEF * min((n - 1u) / gridDim.x, BRIEF_SHARE) : 0u;
+        sm->listed = 0;
+    }
+    u32 q = 0, end = 0, streak = 0; // members in a row that the team did not take
     while (true) {
-        if (threadIdx.x == 0) sm->sh[6] = atomicAdd(queue_head, chunk);
-        __syncthreads();
-        const u32 first = sm->sh[6];
-        __syncthreads();
-        if (first >= n) break;
-        const u32 end = min(n, first + chunk);
-        for (u32 q = first; q < end; ++q) {
-            const u32 m = order ? order[q] : q;
+        if (q == end) {
+            if (!queue) {
+                q = end ? n : blockIdx.x;
+            } else if (q < n) {
+                if (threadIdx.x == 0) sm->sh[6] = atomicAdd(queue_head, chunk);
+                __syncthreads();
+                q = sm->sh[6];
+                __syncthreads();
+            }
+            end = q < n ? (queue ? min(n, q + chunk) : q + 1u) : q;
+        }
+        u32 m;
+        if (q < n) {
+            m = order ? order[q] : q;
+            ++q;
             if (m >= n) continue;
-            const u32 cap = isize[m];
-            u32 p = 0, c = 0, st = INF_OK;
-            if (out_off[m] + cap > out_capacity) {
-                st = INF_OUTPUT_OVERFLOW; // sizes changed since the buffers were planned
-            } else {
-                const u8 *src = in + in_off[m];
-                u8 *to = out + out_off[m];
-                if (!member<NW>(sm, src, in_len[m], to, cap, &p, &c))
-                    st = member_serial<NW>(sm, src, in_len[m], to, cap, &p, &c);
-            }
-            if (threadIdx.x == 0) {
-                status[m] = st;
-                produced[m] = p;
-                crc[m] = st == INF_OK ? c : 0u;
-                const unsigned long long code = st != INF_OK ? 5ull : (p != cap ? 4ull : (c != crc_expect[m] ? 3ull : 0ull));
-                if (code) atomicMin(block_err, ((unsigned long long)m << 8) | code);
-            }
+        } else {
+            __syncthreads();
+            const u32 listed = sm->listed;
+            m = sm->list[0];
+            if (listed > 1) run_listed<NW>(sm, job, listed);
+            if (listed != 1) break;
+            __syncthreads();
+            if (threadIdx.x == 0) sm->listed = sm->brief = 0;
+            streak = 0;
+        }
+        const u32 cap = isize[m], len = in_len[m];
+        const u64 from = in_off[m], to = out_off[m];
+        if (to + cap > out_capacity) { // sizes changed since the buffers were planned
+            if (threadIdx.x == 0) job.put(m, INF_OUTPUT_OVERFLOW, 0, 0);
+            continue;
+        }
+        u32 p = 0, c = 0;
+        if ((streak < 2 || n / NW < gridDim.x) && member<NW>(sm, in + from, len, out + to, cap, &p, &c)) {
+            if (threadIdx.x == 0) job.put(m, INF_OK, p, c);
+            streak = 0;
+            continue;
+        }
+        __syncthreads();
+        clear_marks<NW>(sm); // of what the team decoded before it gave up
+        if (threadIdx.x == 0) sm->list[sm->listed++] = m;
+        __syncthreads();
+        ++streak;
+        if (sm->listed == NW || !sm->brief) {
+            run_listed<NW>(sm, job, sm->listed);
+            streak = 1;
         }
     }
 }

@@ -325,7 +325,7 @@ int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const fr
                   frt_inflate_batch **out, frt_error *err)
 {
     std::vector<uint64_t> plan64(2 * n + 1);
-    std::vector<uint32_t> plan32(2 * n);
+    std::vector<uint32_t> plan32(2 * n + 1);
     uint64_t *in_off = plan64.data(), *out_off = plan64.data() + n;
     uint32_t *in_len = plan32.data(), *cap = plan32.data() + n;
     uint64_t total = 0, in_bytes = 0;
@@ -352,8 +352,8 @@ int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const fr
     DeviceGuard g(c->device);
     std::lock_guard<std::mutex> lk(c->mu);
     cudaStream_t st = c->stream;
-    // one work buffer: in_off | out_off(n+1) | in_len | cap | status | produced | crc
-    size_t work_bytes = 8 * (2 * n + 1) + 4 * 5 * n;
+    // one work buffer: in_off | out_off(n+1) | in_len | cap | the launch's queue head | status | produced | crc
+    size_t work_bytes = 8 * (2 * n + 1) + 4 * (5 * n + 1);
     uint8_t *work = nullptr, *input = nullptr, *output = nullptr;
     uint64_t *d_offsets = nullptr;
     int rc;
@@ -384,16 +384,17 @@ int inflate_batch(frt_codec *c, const uint8_t *batch, size_t batch_len, const fr
     uint64_t *d_out_off = d_in_off + n;
     uint32_t *d_in_len = (uint32_t *)(d_out_off + n + 1);
     uint32_t *d_cap = d_in_len + n;
-    uint32_t *d_status = d_cap + n;
+    uint32_t *d_head = d_cap + n;
+    uint32_t *d_status = d_head + 1;
     uint32_t *d_produced = d_status + n;
     uint32_t *d_crc = d_produced + n;
     cudaError_t e;
     if ((e = cudaMemcpyAsync(input, batch, batch_len, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e, "uploading batch");
     if ((e = cudaMemsetAsync(input + batch_len, 0, 64, st)) != cudaSuccess) return fail(e, "padding batch");
     if ((e = cudaMemcpyAsync(work, plan64.data(), 8 * (2 * n + 1), cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e, "uploading plan");
-    if ((e = cudaMemcpyAsync(d_in_len, plan32.data(), 8 * n, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e, "uploading plan");
+    if ((e = cudaMemcpyAsync(d_in_len, plan32.data(), 4 * plan32.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e, "uploading plan");
     if ((e = frt_launch_inflate_members(input, d_in_off, d_in_len, output, d_out_off, d_cap, d_status, d_produced,
-                                        d_crc, (u32)n, in_bytes, c->tuning, st)) != cudaSuccess)
+                                        d_crc, (u32)n, in_bytes, d_head, c->tuning, st)) != cudaSuccess)
         return fail(e, "launching inflate");
     std::vector<uint32_t> res(3 * n);
     if (n && (e = cudaMemcpyAsync(res.data(), d_status, 12 * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return fail(e, "downloading status");

@@ -2,6 +2,7 @@
 warp a member is quicker than a team: the bytes zlib gives back, the oracle's
 error for a bad member among them, and no longer than the serial form takes."""
 
+import struct
 import zlib
 
 import numpy as np
@@ -80,3 +81,68 @@ def test_short_members_take_no_longer_than_serial(gpu, payload):
     assert team < 1.3 * serial
     eng.run()
     assert eng.finish().status == 0 and np.array_equal(eng.inflated(), raw)
+
+
+def _bam_of(members, count):
+    """A BGZF file of a BAM header's member and `count` members, the given ones
+    (payload, bytes) over and over; and its inflated bytes."""
+    head = b"BAM\x01" + struct.pack("<II", 0, 1) + struct.pack("<I", 5) + b"chr1\0" + struct.pack("<I", 1 << 28)
+    blocks = []
+    for raw, d in [(head, _deflate(head))] + members:
+        blocks.append(b"\x1f\x8b\x08\x04\0\0\0\0\0\xff\x06\0BC\x02\0" + struct.pack("<H", len(d) + 25) + d + struct.pack("<II", zlib.crc32(raw), len(raw)))
+    turns = -(-count // len(members))
+    return (np.frombuffer(blocks[0] + b"".join(blocks[1:] * turns), np.uint8),
+            np.frombuffer(head + b"".join(m[0] for m in members) * turns, np.uint8))
+
+
+def _engine(gpu, bgzf):
+    torch = pytest.importorskip("torch")
+    dev = torch.from_numpy(bgzf.copy()).to("cuda")
+    torch.cuda.synchronize()
+    eng = gpu.BatchEngine(0)
+    eng.bind_bam(dev.data_ptr(), dev.numel())
+    return eng, dev
+
+
+def _short_reads(members):
+    """That many members' worth of whole records."""
+    from fritillaria_gb300 import synth
+
+    raw, ends = synth.raw_bam("short_reads", members * 215, 1, 1 << 28, 3)
+    return [raw[int(ends[k]):int(ends[k + 215])].tobytes() for k in range(0, members * 215, 215)]
+
+
+@pytest.mark.parametrize("count,mem", [(700, 1), (1300, 2), (3000, 1), (3000, 2), (3000, 3), (3000, 8)])
+def test_short_blocks_take_no_longer_than_serial(gpu, count, mem):
+    """Members of 240 to 60 blocks (zlib's memLevel 1 to 3), two and ten a CTA:
+    the default took up to 3.5 times the serial form's time."""
+    bgzf, raw = _bam_of([(r, _deflate(r, mem=mem)) for r in _short_reads(20)], count)
+    eng, _ = _engine(gpu, bgzf)
+    team = eng.time_inflate(gpu.InflateTuning(0, 3, 0, 1), reps=5)[0]
+    serial = eng.time_inflate(gpu.InflateTuning(1, 3, 0, 1), reps=5)[0]
+    assert team < 1.3 * serial
+    eng.run()
+    assert eng.finish().status == 0 and np.array_equal(eng.inflated(), raw)
+
+
+@pytest.mark.parametrize("n", [608, 1300, 4000])
+def test_members_of_short_blocks_among_others(gpu, n):
+    """Through the codec: members of short blocks, of long ones, and short ones;
+    and one bad member of short blocks."""
+    from oracle import oracle
+
+    reads = _short_reads(8)
+    kinds = [(_deflate(reads[k], mem=1 + 7 * (k % 2)), reads[k]) for k in range(8)] + [(_deflate(b"x" * 99), b"x" * 99)]
+    streams = [kinds[k * k % 9] for k in range(n)]
+    data, spans = _file(streams)
+    got, offs = gpu.CudaCodec(0).inflate_batch(data, spans)
+    for i, (_, raw) in enumerate(streams):
+        assert got[offs[i]:offs[i + 1]].tobytes() == raw, i
+    payload, raw = kinds[0]
+    streams[n // 2] = (payload[:-9], raw)
+    data, spans = _file(streams)
+    with pytest.raises(oracle.OracleError) as oe:
+        oracle.inflate_batch(data, spans)
+    with pytest.raises(gpu.FrtError) as ge:
+        gpu.CudaCodec(0).inflate_batch_device(data, spans)
+    assert (ge.value.code, ge.value.offset) == (oe.value.code, oe.value.offset)
