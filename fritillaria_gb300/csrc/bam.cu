@@ -135,7 +135,6 @@ __device__ Seg walk_record(const u8 *buf, u64 len, u64 from, u64 until, u64 msta
 __device__ u64 find_start(const u8 *buf, u64 len, u64 lo, u64 hi, int n_ref)
 {
     const u32 lane = lane_id();
-    hi = min(hi, len); // no record starts past the batch
     const long long A = (long long)(((uintptr_t)(buf + lo) & ~(uintptr_t)3) - (uintptr_t)buf);
     for (long long base = A; base < (long long)hi; base += 512) {
         u32 w0[4], w1[4];
@@ -179,6 +178,7 @@ __device__ u64 find_start(const u8 *buf, u64 len, u64 lo, u64 hi, int n_ref)
 }
 
 constexpr u32 SPEC_WARPS = 8;                          // parts of a member, a warp each
+constexpr u32 SPEC_CTAS = 5;                           // CTAs an SM is to hold: with 4 the record stage of 2,000 members takes 240 us for 225
 constexpr u32 SPEC_PART = 65536 / SPEC_WARPS;          // most bytes of a part
 constexpr u32 SPEC_CAP = (SPEC_PART + 35) / 36;        // most record starts in one
 
@@ -210,10 +210,10 @@ __device__ void spec_member(const u8 *buf, u64 len, const u64 *starts, u32 m, u6
     u64 e = INF64;
     if (lo < hi && hi > start) {
         // the part's lines on their way to L2 while its start is looked for: a
-        // hop of the walk then waits for L2, not for HBM (offsets are the caller's:
-        // none past the batch)
-        for (u64 at = lo + 128ull * lane; at < min(hi, len); at += 128ull * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(buf + at));
-        e = lo <= start ? start : find_start(buf, len, lo, hi, n_ref);
+        // hop of the walk then waits for L2, not for HBM
+        const u64 stop = min(hi, len); // offsets are the caller's: nothing past the batch
+        for (u64 at = lo + 128ull * lane; at < stop; at += 128ull * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(buf + at));
+        e = lo <= start ? start : find_start(buf, len, lo, stop, n_ref);
     }
     if (lane == 0) {
         Seg s{e, 0u, 1, 1};
@@ -266,7 +266,7 @@ __device__ void spec_member_warp(const u8 *buf, u64 len, const u64 *starts, u32 
 {
     const u64 ms = starts[m], me = starts[m + 1];
     u64 e = INF64;
-    if (ms < me && me > start) e = ms <= start ? start : find_start(buf, len, ms, me, n_ref);
+    if (ms < me && me > start) e = ms <= start ? start : find_start(buf, len, ms, min(me, len), n_ref);
     if (lane_id() == 0) {
         Seg s{e, 0u, 1, 1};
         if (e != INF64) s = walk_record(buf, len, e, me, ms, scratch + (size_t)m * FRT_SCAN_CAP, FRT_SCAN_CAP);
@@ -291,7 +291,7 @@ bool spec_by_cta(u64 n, u64 bytes) { return SPEC_MANY * n <= bytes / n; }
 
 // Phase 1.  One CTA per member, or one warp.
 template <bool BY_CTA>
-__global__ void __launch_bounds__(32 * SPEC_WARPS)
+__global__ void __launch_bounds__(32 * SPEC_WARPS, SPEC_CTAS)
 k_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n_members, u64 start, int n_ref, u64 *entry, u32 *count,
            u64 *land, u8 *flags, u16 *scratch, const u64 *start_dev, const int *nref_dev)
 {
@@ -307,7 +307,7 @@ k_bam_spec(const u8 *buf, u64 len, const u64 *starts, u32 n_members, u64 start, 
 // members): segment s owns members [seg[s].m0, seg[s].m0 + seg[s].n) of the
 // per-member arrays and the n + 1 starts at starts + seg[s].m0 + s.
 template <bool BY_CTA>
-__global__ void __launch_bounds__(32 * SPEC_WARPS)
+__global__ void __launch_bounds__(32 * SPEC_WARPS, SPEC_CTAS)
 k_bam_spec_seg(const u8 *buf, const FrtScanSeg *seg, const u32 *seg_of, u32 n_total, int n_ref, const u64 *starts,
                u64 *entry, u32 *count, u64 *land, u8 *flags, u16 *scratch)
 {
