@@ -7,8 +7,9 @@
 // alone.  A DEFLATE block can be decoded from any bit: a decoder started at a
 // wrong place falls into step with the true symbol boundaries after a few
 // dozen codes (on short-read, FASTQ, FASTA and BCF members 1-4% of starts are
-// still out of step after 512 bits, 0.03-0.2% after 1,024).  So the team cuts
-// a block into one segment per lane and goes over it three times:
+// still out of step after 512 bits, 0.03-0.2% after 1,024; codes of one length
+// may never fall into step, see settle).  So the team cuts a block into one
+// segment per lane and goes over it three times:
 //
 //   1. sync:  a lane starts SYNC_BITS before its segment and runs to the
 //             segment's first symbol boundary, its presumed start;
@@ -773,6 +774,112 @@ __device__ __forceinline__ u32 stage_from(Smem<NW> *sm, const u32 *base, u32 wor
     return skew - 32u * w0;
 }
 
+constexpr u32 REPAIRS = 6; // rounds of counting again before all starts may be tried (12 measured 0-20% slower, 8 5%)
+
+// One segment from `start`, counted: its end, from `from` on, how it stopped and
+// its output bytes.
+__device__ __forceinline__ u32 count_segment(u32 stage, u32 tab, u32 off, u32 from, u32 to, u32 start)
+{
+    if (start >= to) return start - from;
+    Walk k;
+    k.start(stage, off + start);
+    const u32 lim = off + to;
+    u32 e, bytes = 0;
+    do {
+        e = k.step(tab);
+        bytes += (e >> 18) & 511u;
+    } while (!(e & 1u) && (k.a < lim || k.b4 != 0u));
+    return (k.a - off - from) | ((e & 1u ? e & 3u : 0u) << 10) | (bytes << 12);
+}
+
+// Maps of a place to a place, sixteen to a word of nibbles; 15 stays 15.
+__device__ __forceinline__ unsigned long long then(unsigned long long first, unsigned long long second, u32 places)
+{
+    unsigned long long m = 0;
+    for (u32 d = 0; d < places; ++d) m |= ((second >> (4u * ((u32)(first >> (4u * d)) & 15u))) & 15ull) << (4u * d);
+    return m | ~0ull << (4u * places);
+}
+
+// The lanes' starts where they do not fall into step (codes of nearly one
+// length: 64 or 128 equally likely symbols).  Counting again proves one lane
+// more a round there, 55 to 216 rounds for a member of 64 KiB.  But a segment
+// begins within a code's length of its boundary, unless a match's extra bits
+// reach over it: so each lane counts its segment from every such place, which
+// maps the place to one in the next segment, and the maps, joined over a warp,
+// take the chain through it in one step.  A warp with a lane that leads to
+// none of the places is followed lane by lane, counting where it has to.
+// Measured on 4,000 members of 64 KiB, inflate alone in ms, counting again only,
+// with this, and the serial variant: 128 symbols, Huffman codes only 24.0, 5.1
+// and 10.4, zlib level 6 19.0, 6.1 and 10.5; 64 symbols 16.2, 5.1 and 10.2, and
+// at level 6, which finds too many matches for this, 6.1, 6.1 and 10.4.
+//
+// Leaves the last lane in sh[3], how it stopped in sh[0] and its end in sh[1];
+// returns the lane's start and, above, its bytes.
+template <int NW>
+__device__ __noinline__ unsigned long long settle(Smem<NW> *sm, u32 off, u32 bitpos, u32 seg, u32 nl, u32 total)
+{
+    const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
+    const u32 tab = smem_u32(sm->tab), stage = smem_u32(sm->stage);
+    const u32 from = bitpos + tid * seg, to = min(bitpos + (tid + 1) * seg, total);
+    u32 places = 1; // as many as the literal/length codes have bits, but for the rarest 64th
+    while (places < 15 && sm->lit.lim[places] < 32768u - 512u) ++places;
+    u32 found[15];
+    unsigned long long map = ~0ull << (4u * places);
+    for (u32 d = 0; d < places; ++d) {
+        u32 next = 15;
+        if (tid < nl) {
+            const u32 r = found[d] = count_segment(stage, tab, off, from, to, from + d);
+            if (tid + 1 < nl && !(r >> 10 & 3u) && (r & 1023u) - seg < places) next = (r & 1023u) - seg;
+        }
+        map |= (unsigned long long)next << (4u * d);
+    }
+#pragma unroll
+    for (u32 k = 1; k < 32; k <<= 1) {
+        const unsigned long long before = __shfl_up_sync(FRT_FULL_MASK, map, k);
+        if (lane >= k) map = then(before, map, places);
+    }
+    const unsigned long long through = __shfl_sync(FRT_FULL_MASK, map, 31), before = __shfl_up_sync(FRT_FULL_MASK, map, 1);
+    if (tid == 0) {
+        sm->sh[2] = bitpos;
+        sm->sh[3] = ~0u;
+    }
+    u32 start = 0, bytes = 0;
+    for (u32 w = 0; w < NW; ++w) {
+        __syncthreads();
+        if (warp != w || sm->sh[3] != ~0u) continue;
+        u32 in = sm->sh[2];
+        const u32 place = in - (bitpos + 32 * w * seg);
+        if (place < places && (through >> (4u * place) & 15u) != 15u) {
+            const u32 mine = lane ? (u32)(before >> (4u * place)) & 15u : place;
+            start = from + mine;
+            bytes = found[mine] >> 12;
+            in = bitpos + 32 * (w + 1) * seg + ((u32)(through >> (4u * place)) & 15u);
+        } else {
+            for (u32 j = 0; j < 32; ++j) {
+                u32 r = 0;
+                if (lane == j) {
+                    r = in - from < places ? found[in - from] : count_segment(stage, tab, off, from, to, in);
+                    start = in;
+                    bytes = r >> 12;
+                }
+                r = __shfl_sync(FRT_FULL_MASK, r, j);
+                in = bitpos + (32 * w + j) * seg + (r & 1023u);
+                if ((r >> 10 & 3u) || 32 * w + j == nl - 1) {
+                    if (lane == 0) {
+                        sm->sh[0] = r >> 10 & 3u;
+                        sm->sh[1] = in;
+                        sm->sh[3] = 32 * w + j;
+                    }
+                    break;
+                }
+            }
+        }
+        if (lane == 0) sm->sh[2] = in;
+    }
+    __syncthreads();
+    return start | ((unsigned long long)bytes << 32);
+}
+
 // A block costs the team some 26 us (its tables, the staging, the barriers) and
 // 0.5 us a kilobit, a warp of the serial form 21 and 15; a CTA has twelve of
 // those, which slow each other down twofold.  So members of several short
@@ -824,7 +931,7 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
             start = k.a - off;
         }
         bool count = mine;
-        u32 E, F;
+        u32 E, F, rounds = 0;
         while (true) { // 2. count
             if (count) {
                 bytes = stop = 0;
@@ -855,6 +962,19 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
             F = __reduce_min_sync(FRT_FULL_MASK, lane < NW ? sm->wb[lane] : 0xffffu); // first lane out of step
             E = min(E, nl - 1u);
             if (F > E) break;
+            // Starts by all places where many lanes are still apart (one in
+            // eight) and next to none ends far over its boundary, in a match:
+            // a warp with one that does takes settle as long as eight rounds.
+            if (++rounds % REPAIRS == 0 && 8 * __syncthreads_count(apart) > nl &&
+                128 * __syncthreads_count(mine && stop == 0 && end - to >= 12u) < nl) {
+                const unsigned long long r = settle<NW>(sm, off, bitpos, seg, nl, total);
+                start = (u32)r;
+                bytes = (u32)(r >> 32);
+                E = sm->sh[3];
+                stop = sm->sh[0];
+                end = sm->sh[1];
+                break;
+            }
             count = apart && tid <= E;
             if (count) start = before;
         }
