@@ -649,7 +649,14 @@ __device__ u32 find_nul_warp(const u8 *rec, u32 q, u32 end)
     return end;
 }
 
-constexpr u32 NUL_ALONE = 64; // bytes of a string a lane looks at before the warp does
+// A string's bytes that a lane looks at before the warp does: NUL_ALONE, then
+// NUL_EACH for each lane of the warp whose string goes on, as the warp takes
+// them one after another.  Record stage of 2,000 members, two strings a record,
+// each lane to its end / the warp from byte 64 on / as it is, us:
+//     100 bytes  312 1652 237    1,000  242 480 189     8,000 1047 779 723
+//     300        199  964 181    2,000  364 386 319    20,000 1165 261 258
+// (64 for each lane 285 at 1,500 bytes for 194, 128 402 at 4,000 for 383).
+constexpr u32 NUL_ALONE = 64, NUL_EACH = 96;
 
 // One aux field at `pos` (aux.rs:301-405) for every lane that is `on`, by the
 // whole warp: the offset just past it, or 0 when malformed.  Fills type and
@@ -660,17 +667,25 @@ __device__ __forceinline__ u32 aux_field(bool on, const u8 *rec, u32 pos, u32 en
     const u32 v = pos + 3;
     const u32 ty = on ? rec[pos + 2] : 0u;
     const bool text = ty == 'Z' || ty == 'H';
-    u32 q = 0;
+    u32 q = 0, lim = 0;
     bool more = false;
     if (text) {
-        const u32 lim = min(end, v + NUL_ALONE);
+        // up to a 16-byte boundary, where what follows goes on in whole loads
+        lim = min(end, v + ((0u - (u32)(uintptr_t)(rec + v)) & 15u) + NUL_ALONE);
         q = find_nul(rec, v, lim);
+        more = q >= lim && lim < end;
+    }
+    const u32 lanes = __popc(__ballot_sync(FRT_FULL_MASK, more));
+    if (more) {
+        const u32 from = lim;
+        lim = min(end, from + NUL_EACH * lanes);
+        q = find_nul(rec, from, lim);
         more = q >= lim && lim < end;
     }
     for (u32 m = __ballot_sync(FRT_FULL_MASK, more); m; m &= m - 1) {
         const u32 l = __ffs(m) - 1;
         const u8 *r = (const u8 *)(uintptr_t)__shfl_sync(FRT_FULL_MASK, (unsigned long long)(uintptr_t)rec, l);
-        const u32 found = find_nul_warp(r, __shfl_sync(FRT_FULL_MASK, v + NUL_ALONE, l), __shfl_sync(FRT_FULL_MASK, end, l));
+        const u32 found = find_nul_warp(r, __shfl_sync(FRT_FULL_MASK, lim, l), __shfl_sync(FRT_FULL_MASK, end, l));
         if (lane_id() == l) q = found;
     }
     if (!on) return 0;
