@@ -385,25 +385,30 @@ __device__ __forceinline__ void flush_some(WarpState *ws, u32 *slot, u32 bitpos,
     }
 }
 
-constexpr u32 kThreads = 1024, kWarps = kThreads / 32; // parts of a parse: 16 of them took half as long again
-constexpr u32 kLinkWarps = 16; // their tables fill the room of `match`
 constexpr u32 kWarm = 512; // bytes a warp parses before its part
 constexpr u32 kOthers = 40;
 
-// A chunk's state: all of an SM's shared memory.
-struct ChunkState {
+// A chunk's state, of at most MAX bytes, for a CTA of THREADS; LINKS of its
+// warps link the prefixes.
+template <u32 THREADS, u32 LINKS, u32 MAX> struct ChunkState {
+    static constexpr u32 kThreads = THREADS, kWarps = THREADS / 32, kLinkWarps = LINKS, kMax = MAX;
     // The latest position + 1 before each one with the same prefix hash (0 none).
-    u16 prev[65536];
+    u16 prev[MAX];
     union {
-        u8 match[65536];                  // match length with it, less 2, 255 for 257 and 258; 0: no match
-        u16 last[kLinkWarps][1u << kHashBits]; // while prev is built: each warp's last position + 1 of a hash
+        u8 match[MAX];                    // match length with it, less 2, 255 for 257 and 258; 0: no match
+        u16 last[LINKS][1u << kHashBits]; // while prev is built: each warp's last position + 1 of a hash
     };
-    u32 inside[2048]; // positions inside a match, but its first
-    u32 first[2048];  // first positions of matches
+    u32 inside[MAX / 32]; // positions inside a match, but its first
+    u32 first[MAX / 32];  // first positions of matches
     u32 start[kWarps], end[kWarps], sums[kWarps];
     u32 other[kWarps][kOthers]; // a warp's matches with a candidate that is not prev: position | candidate << 16
     WarpState tree;
 };
+
+// The shapes a chunk is compressed in.
+using Large = ChunkState<1024, 16, 65536>; // all of an SM's shared memory; 16 parts of a parse took half as long again
+using Medium = ChunkState<256, 4, 8192>;   // four to an SM
+using Small = ChunkState<128, 2, 4096>;    // seven
 
 // Four bytes at p[i], all of them inside the chunk.
 __device__ __forceinline__ u32 load4(const u8 *p, u32 i)
@@ -438,8 +443,9 @@ __device__ __forceinline__ u32 match_length(const u8 *p, u32 q, u32 c, u32 len)
 // with a table of its own (lanes of one hash find each other by match_any);
 // then each hash's last position before every part, and the positions their
 // part had no earlier one for.
-__device__ __forceinline__ void link_prefixes(ChunkState *cs, const u8 *p, u32 len)
+template <class CS> __device__ __forceinline__ void link_prefixes(CS *cs, const u8 *p, u32 len)
 {
+    constexpr u32 kThreads = CS::kThreads, kLinkWarps = CS::kLinkWarps;
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
     const u32 part = (len + 32u * kLinkWarps - 1) / (32u * kLinkWarps) * 32u;
     u16 *last = cs->last[warp % kLinkWarps];
@@ -486,7 +492,8 @@ __device__ __forceinline__ void link_prefixes(ChunkState *cs, const u8 *p, u32 l
 // `c` are its match (L 0: none), `again` whether c is not prev.  It depends on `pos` alone, so parts of the
 // chunk can be parsed apart.  That candidate is prev, or, where prev lies in
 // the step itself, further back along prev (rare: looked at by its bytes).
-__device__ __forceinline__ u32 parse_step(const ChunkState *cs, const u8 *p, u32 len, u32 pos, u32 &m, u32 &L, u32 &c, bool &again)
+template <class CS>
+__device__ __forceinline__ u32 parse_step(const CS *cs, const u8 *p, u32 len, u32 pos, u32 &m, u32 &L, u32 &c, bool &again)
 {
     const u32 lane = lane_id(), q = pos + lane;
     const bool in = q + 3u <= len;
@@ -521,7 +528,7 @@ __device__ __forceinline__ u32 parse_step(const ChunkState *cs, const u8 *p, u32
 }
 
 // Marks the match of L bytes at m in `first` and `inside`, by a warp.
-__device__ __forceinline__ void mark_match(ChunkState *cs, u32 m, u32 L)
+template <class CS> __device__ __forceinline__ void mark_match(CS *cs, u32 m, u32 L)
 {
     // lane 31 marks the first byte, the others the words of [m + 1, m + L): at
     // most 10, most often one
@@ -531,9 +538,9 @@ __device__ __forceinline__ void mark_match(ChunkState *cs, u32 m, u32 L)
     if (lane == 31u || 32u * w < e) atomicOr((lane == 31u ? cs->first : cs->inside) + w, bits);
 }
 
-__device__ __forceinline__ void clear_marks(ChunkState *cs)
+template <class CS> __device__ __forceinline__ void clear_marks(CS *cs)
 {
-    for (u32 i = threadIdx.x; i < 2048u; i += kThreads) cs->inside[i] = cs->first[i] = 0;
+    for (u32 i = threadIdx.x; i < CS::kMax / 32; i += CS::kThreads) cs->inside[i] = cs->first[i] = 0;
     __syncthreads();
 }
 
@@ -543,8 +550,9 @@ __device__ __forceinline__ void clear_marks(ChunkState *cs)
 // a part then does not start where the one before ended (rare), the marks go,
 // the starts are found, each such part again from its right place, and all
 // parts are marked anew.
-__device__ __forceinline__ void parse(ChunkState *cs, const u8 *p, u32 len)
+template <class CS> __device__ __forceinline__ void parse(CS *cs, const u8 *p, u32 len)
 {
+    constexpr u32 kWarps = CS::kWarps;
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x / 32;
     const u32 part = (len + kWarps - 1) / kWarps, from = min(len, warp * part), to = min(len, from + part);
     bool again;
@@ -601,7 +609,8 @@ __device__ __forceinline__ void parse(ChunkState *cs, const u8 *p, u32 len)
 }
 
 // The symbols and extra bits of the match that starts at q.
-__device__ __forceinline__ void match_symbols(const ChunkState *cs, const u8 *p, u32 len, u32 q, u32 &ls, u32 &lex, u32 &lnb,
+template <class CS>
+__device__ __forceinline__ void match_symbols(const CS *cs, const u8 *p, u32 len, u32 q, u32 &ls, u32 &lex, u32 &lnb,
                                               u32 &ds, u32 &dex, u32 &dnb)
 {
     const u32 c = cs->prev[q] - 1u;
@@ -613,8 +622,8 @@ __device__ __forceinline__ void match_symbols(const ChunkState *cs, const u8 *p,
 
 // A symbol's code and extra bits (at most 20, a distance's 28 after them) and
 // their lengths: the match that starts at q, or the literal `byte`.
-template <int MODE>
-__device__ __forceinline__ void symbol_bits(const ChunkState *cs, const u8 *p, u32 len, u32 q, bool match, u32 byte, u32 &v, u32 &nb,
+template <int MODE, class CS>
+__device__ __forceinline__ void symbol_bits(const CS *cs, const u8 *p, u32 len, u32 q, bool match, u32 byte, u32 &v, u32 &nb,
                                             u32 &v2, u32 &nb2)
 {
     const WarpState *ws = &cs->tree;
@@ -668,8 +677,8 @@ struct BitRun {
 
 // Calls f(v, nb, v2, nb2) for each symbol of positions [from, to), in order;
 // `from` is a multiple of 32.
-template <int MODE, class F>
-__device__ __forceinline__ void each_symbol(const ChunkState *cs, const u8 *p, u32 len, u32 from, u32 to, F f)
+template <int MODE, class CS, class F>
+__device__ __forceinline__ void each_symbol(const CS *cs, const u8 *p, u32 len, u32 from, u32 to, F f)
 {
     for (u32 b = from; b < to; b += 32) {
         u32 m = ~cs->inside[b >> 5];
@@ -695,8 +704,10 @@ __device__ __forceinline__ void each_symbol(const ChunkState *cs, const u8 *p, u
 // run of positions, its place from a sum over the team.  Returns the bit past
 // the last, the same in every thread, or 0 where the block with its
 // end-of-block code of `eob` bits would outgrow a BGZF block.
-template <int MODE> __device__ __forceinline__ u32 emit(ChunkState *cs, const u8 *p, u32 len, u32 *slot, u32 bit, u32 eob)
+template <int MODE, class CS>
+__device__ __forceinline__ u32 emit(CS *cs, const u8 *p, u32 len, u32 *slot, u32 bit, u32 eob)
 {
+    constexpr u32 kThreads = CS::kThreads, kWarps = CS::kWarps;
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
     // whole words of marks a thread; the chunk's bytes four at a time
     const u32 per = (len + 32u * kThreads - 1) / (32u * kThreads) * 32u, from = min(len, tid * per), to = min(len, from + per);
@@ -728,25 +739,27 @@ template <int MODE> __device__ __forceinline__ u32 emit(ChunkState *cs, const u8
     return total;
 }
 
-// A CTA per chunk.
+// A CTA per chunk, in one of the three shapes (by_shape).
 //
 // A warp per chunk walked the parse with its hash table, twice: each step a
 // chain of dependent loads through L2, 2,000 cycles, 20 ms for a 64 KiB chunk
 // whatever the number of chunks.  What a step does depends only on where it
 // starts, once every position's earlier positions of its hash are linked: so
 // the links and every position's match length are made by all threads at once,
-// thirty-two warps parse as many parts (parses from different starts fall into
+// the warps parse as many parts (parses from different starts fall into
 // step within a few matches), and counts and codes are taken position by
 // position.  The stream is bit for bit the one-warp form's.  Measured on GB300
 // through compress_batch_device: 454 chunks of short reads (29.6 MB) 19.8 ->
 // 1.64 ms.
-__global__ void __launch_bounds__(kThreads) k_deflate_chunks(const u8 *data, const u64 *bounds, u32 n, u8 *slots,
-                                                             u32 *deflate_len, u32 *crcs)
+template <class CS>
+__global__ void __launch_bounds__(CS::kThreads, 227u * 1024u / (sizeof(CS) + 1024u))
+k_deflate_chunks(const u8 *data, const u64 *bounds, const u32 *which, u8 *slots, u32 *deflate_len, u32 *crcs)
 {
+    constexpr u32 kThreads = CS::kThreads, kWarps = CS::kWarps;
     extern __shared__ __align__(16) unsigned char smem[];
-    ChunkState *cs = (ChunkState *)smem;
+    CS *cs = (CS *)smem;
     WarpState *ws = &cs->tree;
-    const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32, chunk = blockIdx.x;
+    const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32, chunk = which ? which[blockIdx.x] : blockIdx.x;
     const u8 *p = data + bounds[chunk];
     const u32 len = (u32)(bounds[chunk + 1] - bounds[chunk]);
 
@@ -946,6 +959,66 @@ extern "C" size_t frt_framed_size(size_t payload_len, size_t deflate_len)
 
 extern "C" size_t frt_compress_bound(size_t n_chunks) { return n_chunks * (size_t)kMaxBlock; }
 
+namespace {
+constexpr int kShapes = 3;
+
+template <class CS>
+cudaError_t launch_shape(u32 n, const u8 *data, const u64 *bounds, const u32 *which, u8 *slots, u32 *len, u32 *crc, cudaStream_t st)
+{
+    const cudaError_t e = cudaFuncSetAttribute(k_deflate_chunks<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CS));
+    if (e != cudaSuccess) return e;
+    k_deflate_chunks<CS><<<n, CS::kThreads, sizeof(CS), st>>>(data, bounds, which, slots, len, crc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_deflate(int shape, u32 n, const u8 *data, const u64 *bounds, const u32 *which, u8 *slots, u32 *len, u32 *crc,
+                           cudaStream_t st)
+{
+    if (shape == 0) return launch_shape<Large>(n, data, bounds, which, slots, len, crc, st);
+    if (shape == 1) return launch_shape<Medium>(n, data, bounds, which, slots, len, crc, st);
+    return launch_shape<Small>(n, data, bounds, which, slots, len, crc, st);
+}
+
+// The chunks by shape (Large, Medium, Small), counts[] of each; an empty list
+// where all are of one.
+//
+// A chunk of the Large shape has an SM to itself, the quickest for up to one a
+// SM; more of them wait in line, and a short chunk spends most of its time in
+// one warp's tree builder.  Four Medium CTAs or seven Small ones run side by
+// side on an SM.  Measured through compress_batch_device, a warp per chunk /
+// Large / Medium / Small, us:
+//                    152 chunks           500               1,000                20,000
+//     100 bytes  170 116 113 117   177 278 116 118    191  468 182 136    1676  7718 2112 1683
+//   1,000        336 156 151 162   338 442 167 171    360  741 284 190    3230 12916 3758 2530
+//   4,096       1075 207 209 244  1138 617 256 272   1175 1037 417 328   11273 18484 6184 4987
+//   8,192       2244 237 271   -  2247 736 339   -   2452 1245 570   -    (5,000: 7786 5632 2345)
+// so Medium from one chunk a SM on, Small from four.
+std::vector<u32> by_shape(const uint64_t *bounds, size_t n, u32 counts[kShapes])
+{
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    size_t up_to[kShapes] = {0, 0, 0}; // chunks that fit each shape and no smaller one
+    auto smallest = [&](size_t i) {
+        const u64 len = bounds[i + 1] - bounds[i];
+        return len <= Small::kMax ? 2 : len <= Medium::kMax ? 1 : 0;
+    };
+    for (size_t i = 0; i < n; ++i) ++up_to[smallest(i)];
+    const size_t wave = (size_t)sms, fit = up_to[1] + up_to[2];
+    int shape_of[kShapes] = {0, 0, 0}; // of the chunks counted in up_to
+    shape_of[2] = up_to[2] > 4 * wave ? 2 : fit > wave ? 1 : 0;
+    shape_of[1] = (shape_of[2] == 2 ? up_to[1] : fit) > wave ? 1 : 0;
+    counts[0] = counts[1] = counts[2] = 0;
+    for (int k = 0; k < kShapes; ++k) counts[shape_of[k]] += (u32)up_to[k];
+    std::vector<u32> which;
+    if (counts[0] == n || counts[1] == n || counts[2] == n) return which;
+    which.resize(n);
+    u32 at[kShapes] = {0, counts[0], counts[0] + counts[1]};
+    for (size_t i = 0; i < n; ++i) which[at[shape_of[smallest(i)]]++] = (u32)i;
+    return which;
+}
+} // namespace
+
 // DeviceBlockCompressor::compress_batch_device (device.rs:357-371): each
 // range bounds[i]..bounds[i + 1] of the device bytes becomes one framed block,
 // written to the host buffer `out` (out_offsets[i] .. out_offsets[i + 1]); no
@@ -978,14 +1051,18 @@ extern "C" int frt_compress_batch_device(frt_compressor *cp, const uint8_t *data
     DeviceGuardLite g(cp->device);
     std::lock_guard<std::mutex> lk(cp->mu);
     cudaStream_t st = cp->stream;
-    const size_t work = 8 * (n + 1) + 4 * n + 4 * n + (size_t)kSlot * n;
+    u32 counts[kShapes];
+    const std::vector<u32> which = by_shape(bounds, n, counts);
+    const size_t work = 8 * (n + 1) + 4 * n + 4 * n + 4 * which.size() + (size_t)kSlot * n;
     u8 *w = nullptr;
     int rc = dev_alloc((void **)&w, work + 64, st, err);
     if (rc) return rc;
     u64 *d_bounds = (u64 *)w;
     u32 *d_len = (u32 *)(w + 8 * (n + 1));
     u32 *d_crc = d_len + n;
-    u8 *d_slots = (u8 *)(d_crc + n) + ((64 - ((uintptr_t)(d_crc + n) & 63)) & 63);
+    u32 *d_which = which.empty() ? nullptr : d_crc + n;
+    u8 *d_slots = (u8 *)(d_crc + n + which.size());
+    d_slots += (64 - ((uintptr_t)d_slots & 63)) & 63;
     std::vector<u32> lens(n);
     cudaError_t e;
     auto fail = [&](cudaError_t ce, const char *what) {
@@ -994,10 +1071,16 @@ extern "C" int frt_compress_batch_device(frt_compressor *cp, const uint8_t *data
     };
     if ((e = cudaMemcpyAsync(d_bounds, bounds, 8 * (n + 1), cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return fail(e, "uploading the chunk bounds");
-    if ((e = cudaFuncSetAttribute(k_deflate_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkState))) != cudaSuccess)
-        return fail(e, "sizing the deflate");
-    k_deflate_chunks<<<(unsigned)n, kThreads, sizeof(ChunkState), st>>>(data, d_bounds, (u32)n, d_slots, d_len, d_crc);
-    if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "launching the deflate");
+    if (d_which && (e = cudaMemcpyAsync(d_which, which.data(), 4 * which.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess)
+        return fail(e, "uploading the chunks' shapes");
+    u32 at = 0;
+    for (int shape = 0; shape < kShapes; ++shape) {
+        const u32 k = counts[shape];
+        const u32 *list = d_which ? d_which + at : nullptr;
+        if (k && (e = launch_deflate(shape, k, data, d_bounds, list, d_slots, d_len, d_crc, st)) != cudaSuccess)
+            return fail(e, "launching the deflate");
+        at += k;
+    }
     if ((e = cudaMemcpyAsync(lens.data(), d_len, 4 * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return fail(e, "reading the deflate sizes");
