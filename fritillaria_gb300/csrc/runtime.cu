@@ -126,75 +126,6 @@ struct DeviceGuard {
     }
 };
 
-PinnedPool::~PinnedPool()
-{
-    for (const Buffer &b : kept) cudaFreeHost(b.p);
-}
-
-uint8_t *PinnedPool::take(size_t want, size_t *cap)
-{
-    std::lock_guard<std::mutex> lk(mu);
-    size_t best = kept.size();
-    for (size_t i = 0; i < kept.size(); ++i)
-        if (kept[i].cap >= want && (best == kept.size() || kept[i].cap < kept[best].cap)) best = i;
-    if (best == kept.size()) return nullptr;
-    uint8_t *p = kept[best].p;
-    *cap = kept[best].cap;
-    kept.erase(kept.begin() + (ptrdiff_t)best);
-    return p;
-}
-
-void PinnedPool::give(uint8_t *p, size_t cap)
-{
-    if (!p) return;
-    if (cap <= MAX_BYTES) {
-        std::lock_guard<std::mutex> lk(mu);
-        if (kept.size() < MAX_BUFFERS) {
-            kept.push_back({p, cap});
-            return;
-        }
-    }
-    cudaFreeHost(p);
-}
-
-// Host bytes in page-locked memory, so H2D copies run at full link speed; from
-// the codec's pool, and back to it where no copy can still be reading them.
-struct PinnedBytes {
-    std::shared_ptr<PinnedPool> pool;
-    uint8_t *p = nullptr;
-    size_t n = 0, cap = 0;
-    bool idle = true; // no copy in flight
-    ~PinnedBytes() { drop(); }
-    void drop()
-    {
-        if (p && pool && idle) pool->give(p, cap);
-        else if (p) cudaFreeHost(p);
-        p = nullptr;
-    }
-    bool reserve(size_t want)
-    {
-        if (want <= cap) return true;
-        size_t nc = cap ? cap : 1 << 20;
-        while (nc < want) nc *= 2;
-        uint8_t *q = pool ? pool->take(want, &nc) : nullptr;
-        if (!q && cudaMallocHost((void **)&q, nc) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (n) memcpy(q, p, n);
-        drop();
-        p = q;
-        cap = nc;
-        return true;
-    }
-    bool resize(size_t m)
-    {
-        if (!reserve(m)) return false;
-        n = m;
-        return true;
-    }
-};
-
 } // namespace frt
 
 using namespace frt;

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/frt.h"
+#include "pinned.h"
 
 namespace frt {
 
@@ -65,30 +66,6 @@ struct SharedStream {
 SharedStream *stream_create(int device, void *user_stream, frt_error *err);
 SharedStream *stream_retain(SharedStream *s);
 void stream_release(SharedStream *s);
-} // namespace frt
-
-namespace frt {
-// Page-locked host buffers that a codec's readers hand on to the next reader:
-// locking a reader's 16-32 MB took 4 ms each time, more than reading a 25 MB
-// file through it.  At most MAX_BUFFERS of at most MAX_BYTES are kept, the
-// rest is released at once; all go when the codec and its last reader are gone.
-class PinnedPool {
-  public:
-    static constexpr size_t MAX_BUFFERS = 2, MAX_BYTES = 64u << 20;
-    ~PinnedPool();
-    // A kept buffer of at least `want` bytes (the smallest), or null.
-    uint8_t *take(size_t want, size_t *cap);
-    // Keeps p, or releases it.  Nothing may be using it any more.
-    void give(uint8_t *p, size_t cap);
-
-  private:
-    struct Buffer {
-        uint8_t *p;
-        size_t cap;
-    };
-    std::mutex mu;
-    std::vector<Buffer> kept;
-};
 } // namespace frt
 
 struct frt_codec {
