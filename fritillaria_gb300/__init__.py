@@ -286,6 +286,7 @@ def lib():
         "frt_autotune": (C.c_int, [_P, C.c_char_p, C.c_int32, _P, _P]),
         "frt_inflate_variant_count": (C.c_int, []),
         "frt_inflate_variant_info": (C.c_int, [C.c_int32, _P, _P]),
+        "frt_inflate_handed_over": (C.c_int, [C.c_int, _P, _P]),
         "frt_inflate_get_default_tuning": (None, [_P]),
         "frt_inflate_set_default_tuning": (C.c_int, [C.c_int, _P, _P]),
         "frt_inflate_tuning_ctas_per_sm": (C.c_int, [C.c_int, _P]),
@@ -1353,6 +1354,14 @@ def inflate_variants() -> list[dict]:
         _raise(lib().frt_inflate_variant_info(v, C.byref(info), C.byref(err)), err)
         out.append(info.as_dict())
     return out
+
+
+def inflate_handed_over(device: int = 0) -> int:
+    """Members that finished launches of variant 0 left to the serial form since
+    the library was loaded."""
+    n, err = C.c_uint64(), _Err()
+    _raise(lib().frt_inflate_handed_over(device, C.byref(n), C.byref(err)), err)
+    return n.value
 
 
 def inflate_ctas_per_sm(tuning: InflateTuning, device: int = 0) -> int:

@@ -1421,6 +1421,22 @@ extern "C" int frt_inflate_variant_info(int32_t variant, frt_inflate_variant *ou
     return FRT_OK;
 }
 
+extern "C" int frt_inflate_handed_over(int device, uint64_t *members, frt_error *err)
+{
+    if (!members) {
+        frt::set_error(err, FRT_ERR_INVALID_ARGUMENT, 0, 0, 0, 0, nullptr, "null argument");
+        return FRT_ERR_INVALID_ARGUMENT;
+    }
+    const int rc = frt::check_device(device, err);
+    if (rc != FRT_OK) return rc;
+    frt::DeviceGuardLite g(device);
+    unsigned long long n = 0;
+    const cudaError_t e = cudaMemcpyFromSymbol(&n, team::g_handed_over, sizeof n);
+    if (e != cudaSuccess) return frt::cuda_fail(err, e, "reading the handed-over members");
+    *members = n;
+    return FRT_OK;
+}
+
 frt_inflate_tuning frt_inflate_default()
 {
     std::lock_guard<std::mutex> lk(g_tuning_mu);

@@ -1135,6 +1135,8 @@ struct Job {
 
 using Serial = Cfg<9, 7, 1024, 192>;
 
+__device__ unsigned long long g_handed_over; // members the team form left to the serial form
+
 // The `listed` members of sm->list by the serial form, a warp each, in the place
 // of the output and the block's tables.
 template <int NW> __device__ __noinline__ void run_listed(Smem<NW> *sm, const Job &job, u32 listed)
@@ -1151,7 +1153,10 @@ template <int NW> __device__ __noinline__ void run_listed(Smem<NW> *sm, const Jo
     }
     __syncthreads();
     clear_marks<NW>(sm);
-    if (threadIdx.x == 0) sm->listed = 0;
+    if (threadIdx.x == 0) {
+        sm->listed = 0;
+        atomicAdd(&g_handed_over, (unsigned long long)listed);
+    }
     __syncthreads();
 }
 

@@ -640,6 +640,12 @@ int frt_inflate_set_default_tuning(int device, const frt_inflate_tuning *t, frt_
 /* CTAs per SM the tuning runs with on `device`; 0 when it is invalid or does
  * not fit. */
 int frt_inflate_tuning_ctas_per_sm(int device, const frt_inflate_tuning *t);
+/* Members that variant 0's finished launches on `device` left to the serial
+ * form since the library was loaded: invalid ones, those whose codes its
+ * tables do not hold, and, in launches of several members a CTA, those of many
+ * short blocks.  (Launches that go to a serial variant whole, because their
+ * members are short, are not counted.) */
+int frt_inflate_handed_over(int device, uint64_t *members, frt_error *err);
 
 /* ---- batched, device-resident form ---------------------------------------
  * No reference counterpart: the batched launch model.  Members of a whole
