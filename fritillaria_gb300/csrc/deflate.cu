@@ -63,10 +63,9 @@ constexpr ByteCrc make_byte_crc()
 }
 __device__ const ByteCrc g_bcrc = make_byte_crc();
 
-struct WarpState {
-    // the hash table: the last position + 1 of each prefix hash (0 none);
-    // between the passes, the Huffman builder's scratch
-    u32 table[1u << kHashBits];
+constexpr u32 kScratch = 2048; // keys, weights, parents
+struct TreeState {
+    u32 table[kScratch]; // the CRC's byte table, then the Huffman builder's scratch
     u32 ring[kRing];
     u32 lf[286], df[30]; // literal/length and distance symbol counts of the parse
     u16 lcode[286], dcode[30], ccode[19]; // codes, reversed as they are packed
@@ -75,7 +74,7 @@ struct WarpState {
     u32 cf[19];     // counts of the code-length code's symbols
     u32 n_items, hlit, hdist, hclen, dynamic;
 };
-static_assert(sizeof(u32) * (1u << kHashBits) >= 4u * (512 + 1024) + 2u * 1024, "the builder's scratch fits");
+static_assert(sizeof(u32) * kScratch >= 4u * (512 + 1024) + 2u * 1024, "the builder's scratch fits");
 
 __device__ __forceinline__ u32 prefix_hash(u32 b0, u32 b1, u32 b2)
 {
@@ -127,7 +126,7 @@ __device__ __forceinline__ void dist_sym(u32 d, u32 *sym, u32 *ex, u32 *nb)
 
 // Adds each lane's (v, n), n <= 31, at bit `bitpos` + the bits of the lanes
 // below it; returns the new bit position (warp-uniform).
-__device__ __forceinline__ u32 pack(WarpState *ws, u32 bitpos, u32 v, u32 n, u32 lane)
+__device__ __forceinline__ u32 pack(TreeState *ws, u32 bitpos, u32 v, u32 n, u32 lane)
 {
     u32 x = n;
 #pragma unroll
@@ -146,7 +145,7 @@ __device__ __forceinline__ u32 pack(WarpState *ws, u32 bitpos, u32 v, u32 n, u32
 }
 
 // Writes the ring's words [from, to) to the slot and clears them.
-__device__ __forceinline__ void flush(WarpState *ws, u32 *slot, u32 from, u32 to, u32 lane)
+__device__ __forceinline__ void flush(TreeState *ws, u32 *slot, u32 from, u32 to, u32 lane)
 {
     for (u32 w = from + lane; w < to; w += 32u) {
         slot[w] = ws->ring[w % kRing];
@@ -286,7 +285,7 @@ __device__ __forceinline__ u32 cl_extra(u32 sym) { return sym == 16 ? 2u : sym =
 // The dynamic trees from the counts (lf[256] counts the end of block), and
 // whether they beat the fixed codes, their header included (the extra bits
 // of lengths and distances are the same either way).
-__device__ __forceinline__ void build_trees(WarpState *ws, u32 lane)
+__device__ __forceinline__ void build_trees(TreeState *ws, u32 lane)
 {
     u32 *keys = ws->table, *wt = ws->table + 512;
     u16 *parent = (u16 *)(ws->table + 1536);
@@ -377,7 +376,7 @@ __device__ __forceinline__ void build_trees(WarpState *ws, u32 lane)
     __syncwarp();
 }
 
-__device__ __forceinline__ void flush_some(WarpState *ws, u32 *slot, u32 bitpos, u32 &flushed, u32 lane)
+__device__ __forceinline__ void flush_some(TreeState *ws, u32 *slot, u32 bitpos, u32 &flushed, u32 lane)
 {
     if ((bitpos >> 5) - flushed >= kFlush) {
         flush(ws, slot, flushed, flushed + kFlush, lane);
@@ -400,9 +399,9 @@ template <u32 THREADS, u32 LINKS, u32 MAX> struct ChunkState {
     };
     u32 inside[MAX / 32]; // positions inside a match, but its first
     u32 first[MAX / 32];  // first positions of matches
-    u32 start[kWarps], end[kWarps], sums[kWarps];
+    u32 end[kWarps], sums[kWarps], head_bits; // where the warps' parts end; the block header's bits
     u32 other[kWarps][kOthers]; // a warp's matches with a candidate that is not prev: position | candidate << 16
-    WarpState tree;
+    TreeState tree;
 };
 
 // The shapes a chunk is compressed in.
@@ -626,7 +625,7 @@ template <int MODE, class CS>
 __device__ __forceinline__ void symbol_bits(const CS *cs, const u8 *p, u32 len, u32 q, bool match, u32 byte, u32 &v, u32 &nb,
                                             u32 &v2, u32 &nb2)
 {
-    const WarpState *ws = &cs->tree;
+    const TreeState *ws = &cs->tree;
     nb2 = 0;
     if (!match) {
         if (MODE == EMIT_FIXED) fixed_lit(byte, &v, &nb);
@@ -758,7 +757,7 @@ k_deflate_chunks(const u8 *data, const u64 *bounds, const u32 *which, u8 *slots,
     constexpr u32 kThreads = CS::kThreads, kWarps = CS::kWarps;
     extern __shared__ __align__(16) unsigned char smem[];
     CS *cs = (CS *)smem;
-    WarpState *ws = &cs->tree;
+    TreeState *ws = &cs->tree;
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32, chunk = which ? which[blockIdx.x] : blockIdx.x;
     const u8 *p = data + bounds[chunk];
     const u32 len = (u32)(bounds[chunk + 1] - bounds[chunk]);
@@ -846,10 +845,10 @@ k_deflate_chunks(const u8 *data, const u64 *bounds, const u32 *which, u8 *slots,
             }
         }
         flush(ws, slot, flushed, (bitpos + 31u) >> 5, lane);
-        if (lane == 0) cs->start[0] = bitpos;
+        if (lane == 0) cs->head_bits = bitpos;
     }
     __syncthreads();
-    const u32 bit = cs->start[0];
+    const u32 bit = cs->head_bits;
     const bool dyn = ws->dynamic != 0;
     const u32 eob_bits = dyn ? ws->llen[256] : 7u;
     const u32 end = dyn ? emit<EMIT_DYNAMIC>(cs, p, len, slot, bit, eob_bits) : emit<EMIT_FIXED>(cs, p, len, slot, bit, eob_bits);
