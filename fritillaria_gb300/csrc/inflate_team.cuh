@@ -41,14 +41,18 @@
 //
 // Anything out of the ordinary (an invalid or truncated stream, a member over
 // 64 KiB, a code whose tables do not fit) goes to the serial form from the
-// member's start, whose checks and statuses are the reference's.
+// member's start, whose checks and statuses are the reference's; so do, in a
+// launch of many, members of short blocks (BRIEF).
 //
 // Measured on GB300 against the serial form (its tuned shape, the inflate alone):
 // 1M short reads 8.7 -> 2.48 ms (119 GB/s of output), ultra-long reads 6.3 ->
 // 1.26 ms, BCF 3.6 -> 0.78 ms, FASTQ 4.6 -> 1.13 ms, FASTA 3.3 -> 0.63 ms; one
-// short-read member alone 4.4 -> 0.139 ms.  The integer ALUs bound it (ncu: 62%
-// of their peak averaged over phases, 24 warps an SM, 440,000 warp instructions
-// a short-read member; DRAM under 3%).  Twelve warps: ten and eleven measured
+// short-read member alone 4.4 -> 0.139 ms.  No one unit bounds it with the SMs
+// full: 24 warps an SM issue 63% of the time (the ALU pipe 63% busy), and for
+// each instruction a warp waits 1.9 cycles for its own last result, 1.9 at
+// barriers, 1.4 for shared memory (40% of whose wavefronts are bank conflicts),
+// 1.2 for another warp and 0.9 for the ALUs; 403,000 warp instructions a
+// short-read member, DRAM under 3%.  Twelve warps: ten and eleven measured
 // even to 3% slower, sixteen slower (the sync pass grows with the lanes), and
 // 192 to 320 decoding lanes of the twelve warps' 384 0-10% slower.  Two CTAs
 // fill the shared memory; one alone gives two thirds of the rate.
@@ -1161,10 +1165,10 @@ template <int NW> __device__ __noinline__ void run_listed(Smem<NW> *sm, const Jo
 }
 
 // A grid of CTAs that pull members from a queue (`order`, or in their order)
-// through an atomic head, `chunk` a pop; a grid of a CTA for each member, where
-// no order is given, takes one each and no queue (one that is, as the slices of
-// a file still on its way here, shares the SMs with others: a CTA that runs
-// takes members of those that do not yet).
+// through an atomic head, `chunk` a pop.  Where no order is given, a CTA's first
+// member is its own, and the queue begins after those.  (An ordered launch may
+// share the SMs with others, as the slices of a file on its way here do: a CTA
+// that runs takes members in the place of those that do not yet.)
 //
 // A member the team does not take is the serial form's.  Where a CTA has
 // several members to do, such members wait on a list until there is one for
@@ -1183,24 +1187,27 @@ k_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out, const 
     const u32 n = (u32)(n64 < n_cap ? n64 : n_cap);
     if (chunk == 0) chunk = 1;
     const Job job{in, in_off, in_len, out, out_off, isize, crc_expect, status, produced, crc, block_err};
-    const bool queue = order || gridDim.x < n;
     setup<NW>(sm);
     if (threadIdx.x == 0) {
-        sm->brief = queue ? BRIEF * min((n - 1u) / gridDim.x, BRIEF_SHARE) : 0u;
+        sm->brief = n ? BRIEF * min((n - 1u) / gridDim.x, BRIEF_SHARE) : 0u;
         sm->listed = 0;
     }
     u32 q = 0, end = 0, streak = 0; // members in a row that the team did not take
     while (true) {
         if (q == end) {
-            if (!queue) {
-                q = end ? n : blockIdx.x;
+            u32 step = chunk;
+            if (!order && end == 0) {
+                q = blockIdx.x;
+                step = 1;
+            } else if (!order && gridDim.x >= n) {
+                q = n;
             } else if (q < n) {
-                if (threadIdx.x == 0) sm->sh[6] = atomicAdd(queue_head, chunk);
+                if (threadIdx.x == 0) sm->sh[6] = atomicAdd(queue_head, chunk) + (order ? 0u : gridDim.x);
                 __syncthreads();
                 q = sm->sh[6];
                 __syncthreads();
             }
-            end = q < n ? (queue ? min(n, q + chunk) : q + 1u) : q;
+            end = q < n ? min(n, q + step) : q;
         }
         u32 m;
         if (q < n) {
