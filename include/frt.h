@@ -137,7 +137,10 @@ void frt_inflate_batch_free(frt_inflate_batch *b);
 /* A byte source: returns bytes read (0 at end of stream) or -1 on error. */
 typedef int64_t (*frt_read_fn)(void *ctx, uint8_t *buf, size_t cap);
 
-/* DeviceBgzfReader::new(inner, codec).  The codec must outlive the reader. */
+/* DeviceBgzfReader::new(inner, codec).  The codec must outlive the reader.  A
+ * closed reader's page-locked buffer (16-32 MB at the default batch) stays with
+ * the codec for its next reader: at most two, of at most 64 MB each, released
+ * when the codec is destroyed or another buffer cannot be had. */
 int frt_reader_open(frt_read_fn read, void *ctx, frt_codec *codec, frt_reader **out, frt_error *err);
 /* Convenience sources: a caller-owned memory range, or a file path. */
 int frt_reader_open_memory(const uint8_t *data, size_t len, frt_codec *codec, frt_reader **out, frt_error *err);
@@ -600,20 +603,25 @@ void frt_server_release(frt_server *s, uint64_t request);
 /* ---- inflate tuning ----------------------------------------------------------
  * No reference counterpart: the reference launches one fixed kernel shape
  * (crates/fritillaria-cuda/src/backend.rs:178-219).  The member inflate here
- * is compiled in several variants -- literal/length and distance table roots,
- * window buffer and match queue per warp -- and a tuning picks a variant, the
- * warps per CTA (one member per warp), the CTAs per SM and the members a warp
- * takes per pop of the device work queue.  Codecs, engines and servers start
- * from the process-wide default; frt_autotune times candidates on an engine's
- * bound input and caches the winner in a JSON file keyed by device, variant
- * set and workload class. */
+ * is compiled in several variants -- variant 0, the default, gives a member a CTA
+ * (the team form), the others a warp, and differ in literal/length and distance
+ * table roots, window buffer and match queue per warp -- and a tuning picks a
+ * variant, the warps per CTA, the CTAs per SM and the members taken per pop of
+ * the device work queue.  An index names a variant of this library version only:
+ * frt_inflate_variant_info gives its shape, which is what caches go by.
+ * Under variant 0, launches of many short members run a serial variant, and
+ * members of many short blocks are decoded a warp each.
+ * Codecs, engines and servers start from the process-wide default; frt_autotune
+ * times candidates on an engine's bound input and caches the winner in a JSON
+ * file keyed by device, variant set and workload class. */
 typedef struct {
     int32_t variant;        /* index of a compiled variant */
     int32_t warps_per_cta;  /* 1..8; each warp takes the variant's chains of members (variant 0, the
                                team form, gives a member a CTA of its own width whatever this says) */
     int32_t ctas_per_sm;    /* 0: as many as fit */
     int32_t queue_chunk;    /* members per queue pop, 1..64 */
-    int32_t spread_variant; /* -1, or a one-chain variant for small launches: a launch of fewer members
+    int32_t spread_variant; /* -1, or a one-chain variant for small launches (without effect where
+                               `variant` is 0, which gives a member a CTA anyway): a launch of fewer members
                                than one wave of one-warp CTAs holds is made one warp per CTA, and then
                                each member's serial chain bounds it, so a variant with more registers
                                and wider tables does better than the one tuned for throughput */
