@@ -93,6 +93,9 @@ struct Code {
 };
 
 constexpr u32 STAGE_WORDS = 6272; // compressed words of one round: 25 KiB, past the largest default zlib block of the shapes above
+// A lane runs at most one symbol (48 bits) past its segment and loads up to
+// three words ahead.
+constexpr u32 ROUND_BITS = 32u * (STAGE_WORDS - 6);
 constexpr u32 HEAD_BITS = 2304;   // code lengths of a dynamic block: at most 316 symbols of at most 7 bits each
 constexpr u32 MARKS = (OUT_MAX + 16 + 255) / 256 * 8; // words of one mark per output byte, whole groups
 constexpr u32 GROUP_MATCHES = 256 / 3 + 1; // most matches that start in 256 bytes
@@ -901,16 +904,13 @@ constexpr u32 BRIEF = 1500, BRIEF_SHARE = 7;
 
 // One Huffman block from bit `bitpos` (its tables built): bitpos moves past
 // its end-of-block code, pos over its bytes.  `off` is the staged place of bit
-// 0 (stage_from).  False (uniform): the serial form is to take the member.
+// 0 (stage_from), and moves with the stage.  False (uniform): the serial form is to take the member.
 template <int NW>
 __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 words, u32 skew, u32 total, u32 out_at,
-                                             u32 cap, u32 off, u32 &bitpos, u32 &pos, bool last_block)
+                                             u32 cap, u32 &off, u32 &bitpos, u32 &pos, bool last_block)
 {
     constexpr u32 NT = Smem<NW>::NT;
     constexpr u32 SYNC_BITS = 640, MIN_SEG = 192; // 512 and 768, 256 and 384 measured 0-4% slower
-    // a lane runs at most one symbol (48 bits) past its segment and loads up
-    // to three words ahead
-    constexpr u32 ROUND_BITS = 32u * (STAGE_WORDS - 6);
     const u32 block_at = bitpos;
     const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid / 32;
     const u32 tab = smem_u32(sm->tab), stage = smem_u32(sm->stage), out = smem_u32(sm->out), starts = smem_u32(sm->starts);
@@ -1021,11 +1021,7 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
         pos += tot;
         __syncthreads();
         if (how == F_END) {
-            if (!last_block && tid == 0) {
-                sm->hint = bitpos - block_at + (bitpos - block_at) / 16u;
-                const u32 blocks = ++sm->blocks;
-                if (blocks >= 2 && bitpos < blocks * sm->brief && total - bitpos > 2 * sm->brief) sm->fail = 1;
-            }
+            if (!last_block && tid == 0) sm->hint = bitpos - block_at + (bitpos - block_at) / 16u;
             return true;
         }
         off = stage_from<NW>(sm, base, words, skew, bitpos);
@@ -1045,12 +1041,26 @@ __device__ bool member(Smem<NW> *sm, const u8 *in, u32 in_len, u8 *to, u32 cap, 
     const u32 *base = (const u32 *)((u64)in & ~3ull);
     const u32 skew = 8u * (u32)((u64)in & 3ull), total = 8u * in_len;
     const u32 words = (skew + total + 31u) / 32u; // only words that hold payload are read
-    u32 bitpos = 0, pos = 0;
+    u32 bitpos = 0, pos = 0, off = 0;
+    bool coded = false; // the block before: a stored one leaves nothing to wait for
     if (tid == 0) sm->blocks = 0;
     while (true) {
         if (bitpos + 3 > total) return false;
-        const u32 off = stage_from<NW>(sm, base, words, skew, bitpos);
-        if (sm->fail) return false;
+        if (coded) {
+            if (tid == 0) {
+                const u32 blocks = ++sm->blocks;
+                if (blocks >= 2 && bitpos < blocks * sm->brief && total - bitpos > 2 * sm->brief) sm->fail = 1;
+            }
+            __syncthreads();
+            if (sm->fail) return false;
+        }
+        // the words staged do while they hold a stored block's header, or a coded
+        // block like the last one (any header, and a few segments): staging anew
+        // for each, and its barriers, made a short stored block 3 us
+        if (bitpos == 0 || off + bitpos + 64u > ROUND_BITS ||
+            ((bits_at(sm->stage, off + bitpos) & 6u) &&
+             off + bitpos + max(min(total - bitpos, sm->hint), HEAD_BITS + 1024u) > ROUND_BITS))
+            off = stage_from<NW>(sm, base, words, skew, bitpos);
         const u32 v = bits_at(sm->stage, off + bitpos);
         const bool fin = v & 1u;
         const u32 type = (v >> 1) & 3u;
@@ -1061,11 +1071,31 @@ __device__ bool member(Smem<NW> *sm, const u8 *in, u32 in_len, u8 *to, u32 cap, 
             if (at + 4 > in_len) return false;
             const u32 x = bits_at(sm->stage, off + 8u * at), len = x & 0xffffu;
             if (len != (~(x >> 16) & 0xffffu) || at + 4 + len > in_len || len > cap - pos) return false;
-            const u8 *src = in + at + 4;
-            for (u32 i = tid; i < len; i += NT) out[pos + i] = src[i];
+            // from the stage as far as it goes, the rest from HBM
+            const u8 *src = in + at + 4, *near = (const u8 *)sm->stage + (off + 8u * (at + 4)) / 8u;
+            const u32 have = min(len, (ROUND_BITS - (off + 8u * at)) / 8u - 4u);
+            for (u32 i = tid; i < have; i += NT) out[pos + i] = near[i];
+            for (u32 i = have + tid; i < len; i += NT) out[pos + i] = src[i];
             bitpos = 8u * (at + 4 + len);
             pos += len;
+            coded = false;
+            // more of them, up to the last, that lie in the stage whole: the same
+            // by staged bits
+            for (u32 a = off + bitpos; !fin && a + 96u <= ROUND_BITS;) {
+                const u32 *w = sm->stage + (a >> 5), w0 = w[0], w1 = w[1], w2 = w[2];
+                const u32 a2 = (a + 10u) & ~7u, sh = a2 - (a & ~31u);
+                const u32 y = sh < 32u ? __funnelshift_r(w0, w1, sh) : __funnelshift_r(w1, w2, sh - 32u), n = y & 0xffffu;
+                const u32 past = a2 + 32u + 8u * n;
+                if ((__funnelshift_r(w0, w1, a) & 7u) || (y ^ (n << 16)) >> 16 != 0xffffu ||
+                    past > min(ROUND_BITS, off + total) || n > cap - pos)
+                    break;
+                for (u32 i = tid; i < n; i += NT) out[pos + i] = ((const u8 *)sm->stage)[(a2 >> 3) + 4u + i];
+                pos += n;
+                a = past;
+                bitpos = a - off;
+            }
         } else {
+            coded = true;
             u32 nlen = 288, ndist = 32;
             if (type == 2) {
                 u32 a = off + bitpos;

@@ -104,12 +104,12 @@ def _engine(gpu, bgzf):
     return eng, dev
 
 
-def _short_reads(members):
+def _short_reads(members, records=215):
     """That many members' worth of whole records."""
     from fritillaria_gb300 import synth
 
-    raw, ends = synth.raw_bam("short_reads", members * 215, 1, 1 << 28, 3)
-    return [raw[int(ends[k]):int(ends[k + 215])].tobytes() for k in range(0, members * 215, 215)]
+    raw, ends = synth.raw_bam("short_reads", members * records, 1, 1 << 28, 3)
+    return [raw[int(ends[k]):int(ends[k + records])].tobytes() for k in range(0, members * records, records)]
 
 
 @pytest.mark.parametrize("count,mem", [(700, 1), (1300, 2), (3000, 1), (3000, 2), (3000, 3), (3000, 8)])
@@ -146,3 +146,51 @@ def test_members_of_short_blocks_among_others(gpu, n):
     with pytest.raises(gpu.FrtError) as ge:
         gpu.CudaCodec(0).inflate_batch_device(data, spans)
     assert (ge.value.code, ge.value.offset) == (oe.value.code, oe.value.offset)
+
+
+def _flushed(raw, every, level):
+    """Blocks of `every` bytes, an empty stored block after each."""
+    co = zlib.compressobj(level, zlib.DEFLATED, -15, 8)
+    return b"".join(co.compress(raw[a:a + every]) + co.flush(zlib.Z_SYNC_FLUSH) for a in range(0, len(raw), every)) + co.flush()
+
+
+@pytest.mark.parametrize("every", [1, 5, 40, 300, 1000, 7000, 20_000])
+@pytest.mark.parametrize("n", [20, 1000])
+def test_flushed_members_equal_zlib(gpu, every, n):
+    """Short stored blocks and short coded ones in turn, each kind to a member."""
+    raw = _short_reads(1)[0][:60_000 if every >= 300 else 200 * every + 17]
+    kinds = [(_flushed(raw, every, level), raw) for level in (0, 1, 6)]
+    streams = [kinds[k % 3] for k in range(n)]
+    data, spans = _file(streams)
+    got, offs = gpu.CudaCodec(0).inflate_batch(data, spans)
+    for i in range(n):
+        assert got[offs[i]:offs[i + 1]].tobytes() == raw, i
+
+
+@pytest.mark.parametrize("every", [300, 1000, 3000])
+def test_short_stored_blocks_take_no_longer_than_serial(gpu, every):
+    """3,000 members of stored blocks: the default took up to six times the serial
+    form's time."""
+    bgzf, raw = _bam_of([(r, _flushed(r, every, 0)) for r in _short_reads(10, 200)], 3000)
+    eng, _ = _engine(gpu, bgzf)
+    team = eng.time_inflate(gpu.InflateTuning(0, 3, 0, 1), reps=5)[0]
+    serial = eng.time_inflate(gpu.InflateTuning(1, 3, 0, 1), reps=5)[0]
+    assert team < 1.3 * serial
+    eng.run()
+    assert eng.finish().status == 0 and np.array_equal(eng.inflated(), raw)
+
+
+@pytest.mark.parametrize("cut", ["length", "end"])
+def test_a_bad_stored_block_among_short_ones(gpu, cut):
+    from oracle import oracle
+
+    raw = _short_reads(1)[0][:40_000]
+    good = _flushed(raw, 300, 0)
+    for at in (310 * 5, 310 * 70, 310 * 120):  # a block of 300 bytes and an empty one take 310
+        bad = good[:at] if cut == "end" else good[:at + 3] + bytes([good[at + 3] ^ 1]) + good[at + 4:]
+        data, spans = _file([(good, raw), (bad, raw), (good, raw)])
+        with pytest.raises(oracle.OracleError) as oe:
+            oracle.inflate_batch(data, spans)
+        with pytest.raises(gpu.FrtError) as ge:
+            gpu.CudaCodec(0).inflate_batch_device(data, spans)
+        assert (ge.value.code, ge.value.offset) == (oe.value.code, oe.value.offset), at
