@@ -569,7 +569,7 @@ cudaError_t enqueue_inflate(frt_engine *e)
 {
     return frt_launch_inflate_persistent(e->in, e->in_off, e->in_len, e->out, e->out_off, e->isize, e->crc_expect,
                                          e->status, e->produced, e->crc, e->cfg.sort_queue ? e->order : nullptr,
-                                         &e->st->n_members, e->n_cap, e->len, e->out_cap, &e->st->queue_head, (u32)e->grid,
+                                         &e->st->n_members, e->n_cap, e->len, e->out_cap, e->out_cap, &e->st->queue_head, (u32)e->grid,
                                          (unsigned long long *)&e->st->block_err, e->tuning, e->stream);
 }
 
@@ -1213,7 +1213,8 @@ extern "C" int frt_engine_time_inflate(frt_engine *e, const frt_inflate_tuning *
         if ((ce = cudaEventRecord(ev[0], s)) != cudaSuccess) break;
         if ((ce = frt_launch_inflate_persistent(e->in, e->in_off, e->in_len, e->out, e->out_off, e->isize,
                                                 e->crc_expect, e->status, e->produced, e->crc, nullptr,
-                                                &e->st->n_members, k, (u64)((double)e->len * (double)k / (double)e->n_cap), e->out_cap,
+                                                &e->st->n_members, k, (u64)((double)e->len * (double)k / (double)e->n_cap),
+                                                last_off + last_size, e->out_cap,
                                                 &e->st->queue_head, (u32)grid,
                                                 (unsigned long long *)&e->st->block_err, *t, s)) != cudaSuccess)
             break;
@@ -1371,6 +1372,7 @@ int run_host_pipelined(frt_engine *e, const uint8_t *host, size_t len, frt_error
             return bail();
         const u64 m1 = spans.size();
         if (m1 > cap) return bail();
+        const u64 group_from = acc;
         u64 group_bytes = 0;
         for (u64 m = m0; m < m1; ++m) {
             h_in_off[m] = pos + spans[m].payload_start; // discover's payload_start is relative to its buffer
@@ -1419,7 +1421,7 @@ int run_host_pipelined(frt_engine *e, const uint8_t *host, size_t len, frt_error
         if (m1 > m0 &&
             (ce = frt_launch_inflate_persistent(e->in, e->in_off + m0, e->in_len + m0, e->out, e->out_off + m0,
                                                 e->isize + m0, e->crc_expect + m0, e->status + m0, e->produced + m0,
-                                                e->crc + m0, e->order + m0, pp.d_count + k, m1 - m0, group_bytes, e->out_cap,
+                                                e->crc + m0, e->order + m0, pp.d_count + k, m1 - m0, group_bytes, acc - group_from, e->out_cap,
                                                 pp.d_heads + k, (u32)e->grid, (unsigned long long *)(pp.d_errs + k),
                                                 e->tuning, sg)) != cudaSuccess)
             return cuda_fail(err, ce, "launching the inflate");

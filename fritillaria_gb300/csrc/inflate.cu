@@ -1585,28 +1585,31 @@ int ctas_of(std::atomic<int> &known, const frt_inflate_tuning &t)
 //    2,000           202   86 |  213  139 |  223  213 |  227  270 |  241  397
 //    4,000           390  157 |  410  262 |  415  409 |  422  520 |  449  767
 //   40,000          3694 1174 | 3901 1964 | 4042 3077 | 4096 3947 | 4355 5810
-// so the line lies at 190 compressed bytes for each member a CTA has, up to 7.
+// A warp alone takes about 70 ns for a compressed byte and 26 for one of output,
+// so the line lies at 300 bytes for each member a CTA has, up to 7, compressed
+// and three eighths of the inflated ones counted.  (By compressed bytes alone,
+// 4,000 members of 64 KiB of zeros, 100 bytes each, took 4.04 ms for 1.49.)
 constexpr frt_inflate_tuning kShort{1, 3, 0, 1, -1};
-constexpr u64 kShortBytes = 190, kShortShare = 7;
+constexpr u64 kShortBytes = 300, kShortShare = 7;
 
-// `grid` CTAs of a team variant, n members of in_bytes in all.
-bool short_members(u64 grid, u64 n, u64 in_bytes)
+// `grid` CTAs of a team variant, n members of in_bytes and out_bytes in all.
+bool short_members(u64 grid, u64 n, u64 in_bytes, u64 out_bytes)
 {
     const u64 share = grid ? n / grid : 0;
-    return share >= 2 && in_bytes <= n * kShortBytes * std::min(share, kShortShare);
+    return share >= 2 && in_bytes + out_bytes / 8u * 3u <= n * kShortBytes * std::min(share, kShortShare);
 }
 } // namespace
 
 cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                        const u64 *out_off, const u32 *out_cap, u32 *status, u32 *produced,
-                                       u32 *crc, u32 n, u64 in_bytes, u32 *queue_head, const frt_inflate_tuning &tuned,
+                                       u32 *crc, u32 n, u64 in_bytes, u64 out_bytes, u32 *queue_head, const frt_inflate_tuning &tuned,
                                        cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
     frt_inflate_tuning t = tuned;
     if (kVariants[t.variant].team) {
         const int per_sm = ctas_of(g_team_ctas[t.variant], {t.variant, 1, 0, 1, -1});
-        if (per_sm > 0 && short_members((u64)per_sm * (u64)sm_count(), n, in_bytes)) t = kShort;
+        if (per_sm > 0 && short_members((u64)per_sm * (u64)sm_count(), n, in_bytes, out_bytes)) t = kShort;
     }
     u32 unused = 0;
     spread_launch(t, n, &unused);
@@ -1627,13 +1630,13 @@ cudaError_t frt_launch_inflate_members(const u8 *in, const u64 *in_off, const u3
 cudaError_t frt_launch_inflate_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out,
                                           const u64 *out_off, const u32 *isize, const u32 *crc_expect, u32 *status,
                                           u32 *produced, u32 *crc, const u32 *order, const u64 *n_ptr, u64 n_cap,
-                                          u64 in_bytes, u64 out_capacity, u32 *queue_head, u32 grid,
+                                          u64 in_bytes, u64 out_bytes, u64 out_capacity, u32 *queue_head, u32 grid,
                                           unsigned long long *block_err, const frt_inflate_tuning &tuned, cudaStream_t s)
 {
     // n_cap bounds the members (the device count may be lower): fewer than
     // the tuned grid's warps gives a spread launch of n_cap one-warp CTAs
     frt_inflate_tuning t = tuned;
-    if (kVariants[t.variant].team && short_members(grid, n_cap, in_bytes)) {
+    if (kVariants[t.variant].team && short_members(grid, n_cap, in_bytes, out_bytes)) {
         const int per_sm = ctas_of(g_short_ctas, kShort);
         if (per_sm > 0) {
             t = kShort;

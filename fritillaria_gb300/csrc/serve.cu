@@ -337,7 +337,7 @@ int launch_tick(frt_server *sv, std::vector<SrvReq *> &batch, frt_error *err)
     // (a tick of fewer members than the tuned grid has warps is spread one
     // warp per CTA over the SMs by the launcher)
     if ((e = frt_launch_inflate_persistent(sv->files_arena, in_off, in_len, t->arena, out_off, isize, crc, status,
-                                           produced, crc_out, order, n_dev, n, in_bytes, pl.arena_bytes, (u32 *)queue_head,
+                                           produced, crc_out, order, n_dev, n, in_bytes, pl.arena_bytes, pl.arena_bytes, (u32 *)queue_head,
                                            (u32)sv->inflate_grid, block_err, sv->tuning, st)) != cudaSuccess)
         return cuda_fail(err, e, "launching the inflate");
     cudaEventRecord(t->ev_inflated, st);

@@ -194,3 +194,16 @@ def test_a_bad_stored_block_among_short_ones(gpu, cut):
         with pytest.raises(gpu.FrtError) as ge:
             gpu.CudaCodec(0).inflate_batch_device(data, spans)
         assert (ge.value.code, ge.value.offset) == (oe.value.code, oe.value.offset), at
+
+
+def test_short_payloads_of_long_members_stay_with_the_team(gpu):
+    """3,000 members of 60 KB that a few hundred bytes hold: short to read, not to
+    write, and the serial form's time is 1.9 times the team's."""
+    raws = [struct.pack("<IiiBBHHHIiii", 60_000, 0, 5, 2, 9, 0, 0, 0, 0, -1, -1, 0) + b"q\0XXBC" + struct.pack("<I", 60_000 - 42) + bytes([k]) * (60_000 - 42)
+            for k in range(10)]
+    bgzf, raw = _bam_of([(r, _deflate(r)) for r in raws], 3000)
+    eng, _ = _engine(gpu, bgzf)
+    team = eng.time_inflate(gpu.InflateTuning(0, 3, 0, 1), reps=5)[0]
+    assert team < 0.8 * eng.time_inflate(gpu.InflateTuning(1, 3, 0, 1), reps=5)[0]
+    eng.run()
+    assert eng.finish().status == 0 and np.array_equal(eng.inflated(), raw)
