@@ -121,6 +121,7 @@ template <int NW> struct Smem {
     u32 fail, hint;
     u32 brief, blocks; // bits a block below which the member is the serial form's; its blocks so far
     u32 list[NW], listed; // members that wait for the serial form
+    u32 q, q_end, streak; // the CTA's place in the queue, and members in a row that the team did not take
     u16 lsorted[288], dsorted[32];
     u8 lens[320];
 };
@@ -967,9 +968,9 @@ __device__ __forceinline__ bool decode_block(Smem<NW> *sm, const u32 *base, u32 
             E = min(E, nl - 1u);
             if (F > E) break;
             // Starts by all places where many lanes are still apart (one in
-            // eight) and next to none ends far over its boundary, in a match:
+            // eight, and 24: fewer are proven sooner) and next to none ends far over its boundary, in a match:
             // a warp with one that does takes settle as long as eight rounds.
-            if (++rounds % REPAIRS == 0 && 8 * __syncthreads_count(apart) > nl &&
+            if (++rounds % REPAIRS == 0 && 8 * __syncthreads_count(apart) > max(nl, 192u) &&
                 128 * __syncthreads_count(mine && stop == 0 && end - to >= 12u) < nl) {
                 const unsigned long long r = settle<NW>(sm, off, bitpos, seg, nl, total);
                 start = (u32)r;
@@ -1194,6 +1195,39 @@ template <int NW> __device__ __noinline__ void run_listed(Smem<NW> *sm, const Jo
     __syncthreads();
 }
 
+constexpr u32 NONE = 0xffffffffu;
+
+// The CTA's next member, or NONE; by one thread, which keeps its place in
+// shared memory: registers held through a member's decode cost it 1%.
+template <int NW>
+__device__ __forceinline__ u32 next_member(Smem<NW> *sm, const u32 *order, u32 n, u32 *queue_head, u32 chunk)
+{
+    u32 q = sm->q, end = sm->q_end, m = NONE;
+    while (m >= n) { // an order may hold members past the launch's
+        if (q == end) {
+            u32 step = chunk;
+            if (!order && end == 0) {
+                q = blockIdx.x;
+                step = 1;
+            } else if (!order && gridDim.x >= n) {
+                q = n;
+            } else if (q < n) {
+                q = atomicAdd(queue_head, chunk) + (order ? 0u : gridDim.x);
+            }
+            end = q < n ? min(n, q + step) : q;
+            if (q >= n) {
+                m = NONE;
+                break;
+            }
+        }
+        m = order ? order[q] : q;
+        ++q;
+    }
+    sm->q = q;
+    sm->q_end = end;
+    return m;
+}
+
 // A grid of CTAs that pull members from a queue (`order`, or in their order)
 // through an atomic head, `chunk` a pop.  Where no order is given, a CTA's first
 // member is its own, and the queue begins after those.  (An ordered launch may
@@ -1220,40 +1254,21 @@ k_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out, const 
     setup<NW>(sm);
     if (threadIdx.x == 0) {
         sm->brief = n ? BRIEF * min((n - 1u) / gridDim.x, BRIEF_SHARE) : 0u;
-        sm->listed = 0;
+        sm->listed = sm->q = sm->q_end = sm->streak = 0;
     }
-    u32 q = 0, end = 0, streak = 0; // members in a row that the team did not take
     while (true) {
-        if (q == end) {
-            u32 step = chunk;
-            if (!order && end == 0) {
-                q = blockIdx.x;
-                step = 1;
-            } else if (!order && gridDim.x >= n) {
-                q = n;
-            } else if (q < n) {
-                if (threadIdx.x == 0) sm->sh[6] = atomicAdd(queue_head, chunk) + (order ? 0u : gridDim.x);
-                __syncthreads();
-                q = sm->sh[6];
-                __syncthreads();
-            }
-            end = q < n ? min(n, q + step) : q;
-        }
-        u32 m;
-        if (q < n) {
-            m = order ? order[q] : q;
-            ++q;
-            if (m >= n) continue;
-        } else {
-            __syncthreads();
+        if (threadIdx.x == 0) sm->sh[6] = next_member<NW>(sm, order, n, queue_head, chunk);
+        __syncthreads();
+        u32 m = sm->sh[6];
+        if (m == NONE) {
             const u32 listed = sm->listed;
             m = sm->list[0];
             if (listed > 1) run_listed<NW>(sm, job, listed);
             if (listed != 1) break;
             __syncthreads();
-            if (threadIdx.x == 0) sm->listed = sm->brief = 0;
-            streak = 0;
+            if (threadIdx.x == 0) sm->listed = sm->brief = sm->streak = 0;
         }
+        __syncthreads();
         const u32 cap = isize[m], len = in_len[m];
         const u64 from = in_off[m], to = out_off[m];
         if (to + cap > out_capacity) { // sizes changed since the buffers were planned
@@ -1261,19 +1276,23 @@ k_persistent(const u8 *in, const u64 *in_off, const u32 *in_len, u8 *out, const 
             continue;
         }
         u32 p = 0, c = 0;
-        if ((streak < 2 || n / NW < gridDim.x) && member<NW>(sm, in + from, len, out + to, cap, &p, &c)) {
-            if (threadIdx.x == 0) job.put(m, INF_OK, p, c);
-            streak = 0;
+        if ((sm->streak < 2 || n / NW < gridDim.x) && member<NW>(sm, in + from, len, out + to, cap, &p, &c)) {
+            if (threadIdx.x == 0) {
+                job.put(sm->sh[6] != NONE ? sm->sh[6] : sm->list[0], INF_OK, p, c);
+                sm->streak = 0;
+            }
             continue;
         }
         __syncthreads();
         clear_marks<NW>(sm); // of what the team decoded before it gave up
-        if (threadIdx.x == 0) sm->list[sm->listed++] = m;
+        if (threadIdx.x == 0) {
+            sm->list[sm->listed++] = sm->sh[6] != NONE ? sm->sh[6] : sm->list[0];
+            ++sm->streak;
+        }
         __syncthreads();
-        ++streak;
         if (sm->listed == NW || !sm->brief) {
             run_listed<NW>(sm, job, sm->listed);
-            streak = 1;
+            if (threadIdx.x == 0) sm->streak = 1;
         }
     }
 }
